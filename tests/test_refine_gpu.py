@@ -146,6 +146,23 @@ def test_tvl1_denoise_bit_exact_vs_reference(cuda, golden):
     np.testing.assert_array_equal(d.cpu().numpy(), g["out"])
 
 
+@pytest.mark.parametrize("w,h,niters,theta", [(2, 2, 1, 1.0), (65, 3, 7, 1.0), (3, 70, 5, 0.5), (56, 24, 4, 1.0),
+                                              (57, 41, 13, 1.0), (131, 127, 9, 0.7), (321, 203, 30, 1.0)])
+def test_tvl1_denoise_at_region_edges(cuda, w, h, niters, theta):
+    """Images around the regions' sizes and iteration counts around the launches' (odd ones
+    included), bit for bit against the f32 oracle (beta = 0: no expf / powf in the tensor)."""
+    import torch
+    rng = np.random.default_rng(w * 1000 + h)
+    ref = rng.uniform(0, 255, (h, w)).astype(np.float32)
+    depth = rng.uniform(0.5, 5.0, (h, w)).astype(np.float32)
+    d = torch.from_numpy(depth.copy()).to(cuda)
+    ws = torch.empty(M.tvl1_workspace_bytes(w, h) // 8 + 1, dtype=torch.int64, device=cuda)
+    M.tvl1_denoise(torch.from_numpy(ref).to(cuda), d, 0.4, 8.0, M.tvl1_params(niters=niters, theta=theta), ws)
+    torch.cuda.synchronize()
+    want = po.tvl1_denoise(ref, depth, 0.4, 8.0, niters=niters, theta=theta, precision="f32")
+    np.testing.assert_array_equal(d.cpu().numpy(), want)
+
+
 def test_compute3d_matches_reference(cuda):
     import torch
     fr, _, _ = scenes.config_tiny(seed=6, width=40, height=30, n_src=1)
