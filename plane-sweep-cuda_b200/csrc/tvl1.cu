@@ -10,6 +10,7 @@
 // floats.
 #include <math.h>
 
+#include "blocked.cuh"
 #include "common.cuh"
 #include "proj.cuh"
 
@@ -60,21 +61,18 @@ struct Bufs {
     float *out, *R_out, *Px_out, *Py_out;
     int w, h;
     int iters;          // iterations of this launch
-    int halo;           // at least iters, even
+    int halo;           // block_halo(iters)
     int first;          // 1: this launch starts the run
     float sigma_first, sigma_p, tau, theta, lambda, sigma, znear, inputscale;
 };
 
-// `iters` iterations in one launch.  A CTA holds a region of BW columns x
-// (RPT x warps) rows in registers: lane l has columns 2l and 2l + 1 of its
-// warp's RPT rows (primal, px, py, r and the data term; the tensor, as the
-// doubles the update wants, in shared memory).  Neighbours in x come by warp
-// shuffles, in y from the thread's own rows or, across warps, from one row per
-// warp and direction in shared memory, so an iteration is two barriers and no
-// global access.  An iteration reads one cell further on every side, so of the
-// region only the cells at least `halo` from its rim are stored: the
-// neighbouring regions compute the rest.  Nothing that another CTA reads is
-// written in place (primal, p and r are double-buffered).
+// `iters` iterations in one launch on the regions of blocked.cuh: primal, px,
+// py, r and the data term in registers, the tensor, as the doubles the update
+// wants, in shared memory.  Neighbours in x come by warp shuffles, in y from
+// the thread's own rows or, across warps, from one row per warp and direction
+// in shared memory, so an iteration is two barriers and no global access.
+// Nothing that another CTA reads is written in place (primal, p and r are
+// double-buffered).
 //
 // What bounds it: instruction issue and the FP64 and conversion pipes (about
 // 120 instructions, 30 of them FP64 and 6 conversions, per cell and
@@ -82,7 +80,7 @@ struct Bufs {
 // iteration was bound by that chain of launch, loads and barriers alone: 7.2 us
 // an iteration at 640x480, of which the IEEE double square root and divisions
 // of the projections were a third; 3.0 us in this form (B200).
-constexpr int BW = 64, RPT = 2, MAXWARPS = 32;
+constexpr int BW = kBlockW, RPT = kBlockRows, MAXWARPS = 32;
 
 template <bool THETA1>
 __global__ void __launch_bounds__(32 * MAXWARPS) tvl1_block_kernel(Bufs b)
@@ -224,35 +222,6 @@ __global__ void tvl1_finish_kernel(const float *__restrict__ in, int n, float sc
         out[i] = in[i] * scale + znear;
 }
 
-// Iterations per launch (even) and warps per CTA.  More of either means fewer
-// launches or less halo, but also more cells on the busiest SM.  Measured on
-// the B200 over 97x73 to 1242x375, a launch takes about 4.2 us plus 0.08 us for
-// every iteration and warp on the busiest SM, within 10%; the pair with the
-// smallest such sum is taken (640x480: 4 iterations, 24 warps, 298 us per 100
-// iterations against 324 us for 14 warps and 389 us for 2 iterations;
-// 320x240: 6 and 12, 176 us; 1242x375: 400 us).
-struct Plan {
-    int iters, warps;
-};
-
-Plan block_plan(int w, int h, int niters)
-{
-    Plan best{2, MAXWARPS};
-    double cost = 1e30;
-    for (int k = 2; k <= 10; k += 2)
-        for (int warps = k / RPT * 2 + 2; warps <= MAXWARPS; ++warps) {
-            const int rows = ceil_div(h, RPT * warps - 2 * k);
-            if (rows > 65535) continue;   // the grid's y extent
-            const long tiles = (long)ceil_div(w, BW - 2 * k) * rows;
-            const double c = ceil_div(niters, k) * (4.2 + 0.08 * k * warps * (double)((tiles + kSMs - 1) / kSMs));
-            if (c < cost) {
-                cost = c;
-                best = Plan{k, warps};
-            }
-        }
-    return best;
-}
-
 struct Layout {
     float *T11, *T12, *T22, *D[2], *R[2], *Px[2], *Py[2];
     size_t bytes;
@@ -315,13 +284,17 @@ int tvl1_run(int w, int h, const float *ref255, float *depth, float znear, float
     // first dual step uses sigma + 1 (planesweep.cpp:347)
     b.sigma_first = (float)(1.0 + (double)prm->sigma);
     b.sigma_p = (float)(double)prm->sigma;
-    const Plan plan = block_plan(w, h, prm->niters);
+    // Measured on the B200 over 97x73 to 1242x375: 4.2 us a launch plus 0.08 us an
+    // iteration and warp, within 10% (640x480: 4 iterations and 24 warps, 284 us
+    // per 100 iterations, against 324 us for 4 and 14 and 389 us for 2 and 24;
+    // 320x240: 6 and 12, 176 us; 1242x375: 400 us)
+    const BlockPlan plan = block_plan(w, h, prm->niters, MAXWARPS, 4.2, 0.08);
     const size_t smem = (size_t)3 * RPT * plan.warps * 32 * sizeof(double2);
     auto kernel = b.theta == 1.f ? tvl1_block_kernel<true> : tvl1_block_kernel<false>;
     MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     for (int it = 0; it < prm->niters; it += b.iters) {
         b.iters = min(plan.iters, prm->niters - it);
-        b.halo = (b.iters + 1) & ~1;
+        b.halo = block_halo(b.iters);
         b.first = it == 0;
         b.in = L.D[cur];
         b.R_in = L.R[cur];
@@ -331,8 +304,7 @@ int tvl1_run(int w, int h, const float *ref255, float *depth, float znear, float
         b.R_out = L.R[cur ^ 1];
         b.Px_out = L.Px[cur ^ 1];
         b.Py_out = L.Py[cur ^ 1];
-        const dim3 g(ceil_div(w, BW - 2 * b.halo), ceil_div(h, RPT * plan.warps - 2 * b.halo));
-        MVS_TRY_CUDA(launch_dependent(kernel, g, dim3(32 * plan.warps), smem, st, b));
+        MVS_TRY_CUDA(launch_dependent(kernel, block_grid(w, h, b.iters, plan.warps), dim3(32 * plan.warps), smem, st, b));
         cur ^= 1;
     }
     tvl1_finish_kernel<<<min(ceil_div(n, 256), 8 * kSMs), 256, 0, st>>>(L.D[cur], n, zfar - znear, znear, depth);

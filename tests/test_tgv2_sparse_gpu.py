@@ -56,6 +56,14 @@ def test_sparse_tensor_vs_reference(cuda, golden):
     assert rel.max() <= 1e-5, rel.max()
 
 
+@pytest.mark.parametrize("w,h,niters", [(56, 24, 4), (57, 41, 13), (65, 3, 7), (131, 127, 9), (321, 203, 21)])
+def test_sparse_at_region_edges_bit_exact_vs_oracle(cuda, w, h, niters):
+    """Images around the regions' sizes and iteration counts around the launches'."""
+    ref, depth, sparse = sparse_case(w + h, w, h)
+    out = run_sparse(cuda, ref, depth, sparse, 6.0, niters)
+    np.testing.assert_array_equal(out, po.tgv_sparse(ref, depth, sparse, 6.0, niters, precision="f32"))
+
+
 @pytest.mark.parametrize("w,h,niters", [(1, 17, 9), (17, 1, 9), (2, 2, 5), (33, 7, 12), (97, 61, 30)])
 def test_sparse_ragged_sizes_bit_exact_vs_oracle(cuda, w, h, niters):
     ref, depth, sparse = sparse_case(w * 131 + h, w, h)
