@@ -174,7 +174,8 @@ typedef struct mvs_tgv2_params {
 #define MVS_TGV2_STOP_WINDOW_DEFAULT 5
 #define MVS_TGV2_STOP_WINDOW_MAX 16
 
-#define MVS_TGV2_ITER_AUTO 0     /* the fastest measured form: as MVS_TGV2_ITER_LAUNCH */
+#define MVS_TGV2_ITER_AUTO 0     /* the fastest measured form for the size: several iterations per
+                                    launch on small frames, else as MVS_TGV2_ITER_LAUNCH */
 #define MVS_TGV2_ITER_LAUNCH 1   /* one fused launch per iteration (dependent launches, state in
                                     L2), energy checks and the stopping test on the device */
 #define MVS_TGV2_ITER_PERSISTENT 2 /* one cooperative launch per linearisation with the state on

@@ -28,9 +28,11 @@ inline dim3 block_grid(int w, int h, int iters, int warps)
 
 // More iterations or more warps mean fewer launches or less halo, but also
 // more cells on the busiest SM.  A launch takes about `launch_us` plus
-// `warp_us` for every iteration and warp on the busiest SM (both measured, see
-// the callers); the pair with the smallest such sum for the run is taken.
-inline BlockPlan block_plan(int w, int h, int niters, int max_warps, double launch_us, double warp_us)
+// `warp_us` for every iteration and warp on the busiest SM, its loads counting
+// as `load_iters` iterations (all measured, see the callers); the pair with the
+// smallest such sum for the run is taken, and that sum returned in `us`.
+inline BlockPlan block_plan(int w, int h, int niters, int max_warps, double launch_us, double warp_us,
+                            int load_iters = 0, double *us = nullptr)
 {
     BlockPlan best{2, max_warps};
     double cost = 1e30;
@@ -39,12 +41,13 @@ inline BlockPlan block_plan(int w, int h, int niters, int max_warps, double laun
             const dim3 g = block_grid(w, h, k, warps);
             if (g.y > 65535u) continue;
             const double tiles = ceil((double)g.x * g.y / kSMs);
-            const double c = ceil_div(niters, k) * (launch_us + warp_us * k * warps * tiles);
+            const double c = ceil_div(niters, k) * (launch_us + warp_us * (k + load_iters) * warps * tiles);
             if (c < cost) {
                 cost = c;
                 best = BlockPlan{k, warps};
             }
         }
+    if (us) *us = cost;
     return best;
 }
 

@@ -255,6 +255,14 @@ __device__ __forceinline__ double proj_norm(double s) { return s > 1.0 ? (double
 // exactly +-1 in IEEE arithmetic (NaN stays NaN, as in the division).
 __device__ __forceinline__ float proj_unit(float r) { return fabsf(r) > 1.f ? copysignf(1.f, r) : r; }
 
+// proj_unit as two instructions: NaN stays NaN.
+__device__ __forceinline__ float clamp_unit(float r)
+{
+    asm("min.NaN.f32 %0, %0, %1;" : "+f"(r) : "f"(1.f));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(r) : "f"(-1.f));
+    return r;
+}
+
 // (float)(v / d) for the reference's projections with d = proj_norm(s): the
 // square root and the FP64 divisions sit behind real branches, so warps whose
 // projections are all the identity skip them.
@@ -624,6 +632,267 @@ __global__ void __launch_bounds__(TX *TY) iteration_kernel(IterBufs b)
     b.Qx_out[i] = qx;
     b.Qy_out[i] = qy;
     b.Qz_out[i] = qz;
+}
+
+// ---- several iterations per launch ------------------------------------------------
+
+struct BlockBufs {
+    const IterCtl *ctl;   // null: no stopping test
+    const float *T11, *T12, *T22, *u0, *It, *Iu;
+    const float *u_in, *u1x_in, *u1y_in, *ubar_in, *u1xbar_in, *u1ybar_in, *Px_in, *Py_in, *Qx_in, *Qy_in, *Qz_in,
+        *r_in;
+    float *u_out, *u1x_out, *u1y_out, *ubar_out, *u1xbar_out, *u1ybar_out, *Px_out, *Py_out, *Qx_out, *Qy_out, *Qz_out,
+        *r_out;
+    int w, h, V;
+    int iters, halo;   // iterations of this launch, block_halo(iters)
+    int first;         // 1: the linearisation precedes this launch
+    float lambda, alpha0, alpha1, tau, sigma;
+};
+
+constexpr int TGW = 12;   // warps per CTA at most
+constexpr size_t kSmemMax = 227 * 1024;   // shared memory of a CTA
+// shared memory per warp: T11, T12, T22, u0, u, u1x, u1y and the views' r, It, Iu
+// of each cell, and the rows exchanged with its neighbours
+constexpr size_t block_warp_bytes(int V)
+{
+    return (size_t)kBlockRows * 64 * (7 + 3 * view_stride(V)) * sizeof(float) + 7 * 32 * sizeof(float2);
+}
+constexpr size_t kBlockBytes = 7 * 32 * sizeof(float2);   // the exchange rows outside the region
+
+// `iters` iterations (planesweep.cpp:485-509) in one launch on the regions of
+// blocked.cuh.  ubar, vbar, p and q stay in registers; T, u0, u, v and the
+// views' r, It and Iu (VS of them, V rounded up to a multiple of 4) in shared
+// memory, each cell used by one thread only.  Neighbours in x come by warp shuffles, in y from the thread's own rows
+// or, across warps, from shared rows.
+//
+// What bounds it: instruction issue of two to three warps per scheduler (the
+// views' state fills the shared memory at 12 warps), and the launch with its
+// loads.  It and Iu read from L2 in every iteration instead, for twice the
+// warps, was slower: 5.3 against 4.4 us an iteration at 320x240 with 4 views,
+// 14.3 against 14.3 at 640x480 with 8.
+template <int VS>
+__global__ void __launch_bounds__(32 * TGW) tgv2_block_kernel(BlockBufs b)
+{
+    constexpr int RPT = kBlockRows, BW = kBlockW;
+    extern __shared__ float4 sR[];   // r: [VS / 4][rows][column of the pair][32]; It, Iu alike (sI)
+    const int w = b.w, h = b.h, V = b.V, K = b.halo;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int rows = RPT * warps, plane = rows * 32;
+    float4 *sI = sR + (VS / 4) * rows * 64;
+    float2 *sF = reinterpret_cast<float2 *>(sI + 2 * (VS / 4) * rows * 64);   // [7][rows][32]: T11, T12, T22, u0, u, u1x, u1y
+    // rows read by neighbouring warps: ubar, vbar of each warp's first row; px,
+    // py, qy, qz of its last (zeros outside the region: they only reach halo cells)
+    float2 *sEx = sF + 7 * plane;
+    const int ex = 32 * (warps + 1);
+    auto top = [&](int k, int wp) -> float2 & { return sEx[k * ex + wp * 32 + lane]; };
+    auto bot = [&](int k, int wp) -> float2 & { return sEx[(3 + k) * ex + wp * 32 + lane]; };
+    const int xa = (int)blockIdx.x * (BW - 2 * K) - K + 2 * lane;
+    const int y0 = (int)blockIdx.y * (rows - 2 * K) - K + RPT * warp;
+    bool in[RPT][2];
+#pragma unroll
+    for (int j = 0; j < RPT; ++j)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) in[j][c] = xa + c >= 0 && xa + c < w && y0 + j >= 0 && y0 + j < h;
+    auto load2 = [&](const float *src, int j) {
+        const size_t i = (size_t)(y0 + j) * w + xa;
+        return make_float2(in[j][0] ? src[i] : 0.f, in[j][1] ? src[i + 1] : 0.f);
+    };
+    if (b.first) wait_for_previous_grid();   // the linearisation is complete
+    {
+        // constant through a linearisation: read before the wait in its later launches
+        const float *const src[4] = {b.T11, b.T12, b.T22, b.u0};
+#pragma unroll
+        for (int j = 0; j < RPT; ++j)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) sF[k * plane + (RPT * warp + j) * 32 + lane] = load2(src[k], j);
+#pragma unroll
+        for (int j = 0; j < RPT; ++j)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const size_t i = (size_t)(y0 + j) * w + (xa + c);
+                const float4 *t4 = reinterpret_cast<const float4 *>(b.It + i * VS);
+                const float4 *d4 = reinterpret_cast<const float4 *>(b.Iu + i * VS);
+#pragma unroll
+                for (int q = 0; q < VS / 4; ++q) {
+                    sI[((2 * q * rows + RPT * warp + j) * 2 + c) * 32 + lane] =
+                        in[j][c] ? t4[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    sI[(((2 * q + 1) * rows + RPT * warp + j) * 2 + c) * 32 + lane] =
+                        in[j][c] ? d4[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+    }
+    if (!b.first) wait_for_previous_grid();   // dependent launch: the previous iterations are complete
+    allow_next_grid();
+    if (b.ctl && b.ctl->done) return;   // the run stopped at an earlier energy check
+    float2 ub[RPT], vxb[RPT], vyb[RPT];
+    float px[RPT][2], py[RPT][2], qx[RPT][2], qy[RPT][2], qz[RPT][2];
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) {
+        const int at = (RPT * warp + j) * 32 + lane;
+        sF[4 * plane + at] = load2(b.u_in, j);
+        sF[5 * plane + at] = load2(b.u1x_in, j);
+        sF[6 * plane + at] = load2(b.u1y_in, j);
+        ub[j] = load2(b.ubar_in, j);
+        vxb[j] = load2(b.u1xbar_in, j);
+        vyb[j] = load2(b.u1ybar_in, j);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const size_t i = (size_t)(y0 + j) * w + (xa + c);
+            px[j][c] = in[j][c] ? b.Px_in[i] : 0.f;
+            py[j][c] = in[j][c] ? b.Py_in[i] : 0.f;
+            qx[j][c] = in[j][c] ? b.Qx_in[i] : 0.f;
+            qy[j][c] = in[j][c] ? b.Qy_in[i] : 0.f;
+            qz[j][c] = in[j][c] ? b.Qz_in[i] : 0.f;
+            const float4 *r4 = reinterpret_cast<const float4 *>(b.r_in + i * VS);
+#pragma unroll
+            for (int q = 0; q < VS / 4; ++q)
+                sR[((q * rows + RPT * warp + j) * 2 + c) * 32 + lane] =
+                    in[j][c] ? r4[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    if (warp == 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) top(k, warps) = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) bot(k, 0) = make_float2(0.f, 0.f);
+    }
+    const bool right0 = xa + 1 <= w - 1, right1 = xa + 2 <= w - 1;   // has a right neighbour
+    const float a1s = b.alpha1 * b.sigma, a0s = b.alpha0 * b.sigma, sl = b.sigma * b.lambda;
+    for (int k = 0; k < b.iters; ++k) {
+        top(0, warp) = ub[0];
+        top(1, warp) = vxb[0];
+        top(2, warp) = vyb[0];
+        // r and prodsum (TGV2_updateR_kernel, TGV2_kernels.cu:87-105), views in order
+        float prodsum[RPT][2];
+#pragma unroll
+        for (int j = 0; j < RPT; ++j) {
+            const int at = (RPT * warp + j) * 32 + lane;
+            const float2 uo = sF[4 * plane + at], uz = sF[3 * plane + at];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float du = c ? uo.y - uz.y : uo.x - uz.x;
+                float4 t[VS / 4], d[VS / 4];
+#pragma unroll
+                for (int q = 0; q < VS / 4; ++q) {
+                    t[q] = sI[((2 * q * rows + RPT * warp + j) * 2 + c) * 32 + lane];
+                    d[q] = sI[(((2 * q + 1) * rows + RPT * warp + j) * 2 + c) * 32 + lane];
+                }
+                float ps = 0.f;
+#pragma unroll
+                for (int q = 0; q < VS / 4; ++q) {
+                    float4 &rq = sR[((q * rows + RPT * warp + j) * 2 + c) * 32 + lane];
+                    float4 r = rq;
+                    r.x = clamp_unit(r.x + sl * (t[q].x + du * d[q].x));
+                    ps += r.x * d[q].x;
+                    if (q < VS / 4 - 1 || 4 * q + 1 < V) {
+                        r.y = clamp_unit(r.y + sl * (t[q].y + du * d[q].y));
+                        ps += r.y * d[q].y;
+                    }
+                    if (q < VS / 4 - 1 || 4 * q + 2 < V) {
+                        r.z = clamp_unit(r.z + sl * (t[q].z + du * d[q].z));
+                        ps += r.z * d[q].z;
+                    }
+                    if (q < VS / 4 - 1 || 4 * q + 3 < V) {
+                        r.w = clamp_unit(r.w + sl * (t[q].w + du * d[q].w));
+                        ps += r.w * d[q].w;
+                    }
+                    rq = r;
+                }
+                prodsum[j][c] = ps;
+            }
+        }
+        // p and q of one row; du, dvx, dvy: the row below
+        auto pq_row = [&](int j, float2 du, float2 dvx, float2 dvy) {
+            const float nu = __shfl_down_sync(0xffffffffu, ub[j].x, 1);
+            const float nvx = __shfl_down_sync(0xffffffffu, vxb[j].x, 1);
+            const float nvy = __shfl_down_sync(0xffffffffu, vyb[j].x, 1);
+            const bool down = y0 + j + 1 <= h - 1;
+            const float uc[2] = {ub[j].x, ub[j].y}, vxc[2] = {vxb[j].x, vxb[j].y}, vyc[2] = {vyb[j].x, vyb[j].y};
+            const float ur[2] = {right0 ? uc[1] : uc[0], right1 ? nu : uc[1]};
+            const float vxr[2] = {right0 ? vxc[1] : vxc[0], right1 ? nvx : vxc[1]};
+            const float vyr[2] = {right0 ? vyc[1] : vyc[0], right1 ? nvy : vyc[1]};
+            const float ud[2] = {down ? du.x : uc[0], down ? du.y : uc[1]};
+            const float vxd[2] = {down ? dvx.x : vxc[0], down ? dvx.y : vxc[1]};
+            const float vyd[2] = {down ? dvy.x : vyc[0], down ? dvy.y : vyc[1]};
+            const float2 *tr = sF + (RPT * warp + j) * 32 + lane;
+            const float2 f11 = tr[0], f12 = tr[plane], f22 = tr[2 * plane];
+            p_pair(uc, ur, ud, vxc, vyc, make_double2(f11.x, f11.y), make_double2(f12.x, f12.y),
+                   make_double2(f22.x, f22.y), a1s, px[j], py[j]);
+            q_pair(vxc, vxr, vxd, vyc, vyr, vyd, a0s, qx[j], qy[j], qz[j]);
+        };
+        // primal step (TGV2_updateU_tensor_weighed_kernel, TGV2_kernels.cu:300-338) of one row; upx, upy, uqy, uqz: the row above
+        auto u_row = [&](int j, float2 upx, float2 upy, float2 uqy, float2 uqz) {
+            const float npx = __shfl_up_sync(0xffffffffu, px[j][1], 1), npy = __shfl_up_sync(0xffffffffu, py[j][1], 1);
+            const float nqx = __shfl_up_sync(0xffffffffu, qx[j][1], 1), nqz = __shfl_up_sync(0xffffffffu, qz[j][1], 1);
+            const bool l = xa > 0, up = y0 + j > 0;
+            const float pxl[2] = {l ? npx : px[j][0], px[j][0]}, pyl[2] = {l ? npy : py[j][0], py[j][0]};
+            const float qxl[2] = {l ? nqx : qx[j][0], qx[j][0]}, qzl[2] = {l ? nqz : qz[j][0], qz[j][0]};
+            const float pxu[2] = {up ? upx.x : px[j][0], up ? upx.y : px[j][1]};
+            const float pyu[2] = {up ? upy.x : py[j][0], up ? upy.y : py[j][1]};
+            const float qyu[2] = {up ? uqy.x : qy[j][0], up ? uqy.y : qy[j][1]};
+            const float qzu[2] = {up ? uqz.x : qz[j][0], up ? uqz.y : qz[j][1]};
+            float2 *fr = sF + (RPT * warp + j) * 32 + lane;
+            const float2 f11 = fr[0], f12 = fr[plane], f22 = fr[2 * plane];
+            const float2 ou = fr[4 * plane], ox = fr[5 * plane], oy = fr[6 * plane];
+            float un[2], xn[2], yn[2];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float t11 = c ? f11.y : f11.x, t12 = c ? f12.y : f12.x, t22 = c ? f22.y : f22.x;
+                const float cpx = px[j][c], cpy = py[j][c];
+                un[c] = (c ? ou.y : ou.x) - b.tau * (-b.alpha1 * (t11 * (cpx - pxl[c]) + t12 * (cpy - pyl[c]) +
+                                                                  t12 * (cpx - pxu[c]) + t22 * (cpy - pyu[c])) +
+                                                     b.lambda * prodsum[j][c]);
+                xn[c] = (c ? ox.y : ox.x) - b.tau * (-b.alpha1 * (t11 * cpx + t12 * cpy) -
+                                                     b.alpha0 * (qx[j][c] - qxl[c] + qz[j][c] - qzu[c]));
+                yn[c] = (c ? oy.y : oy.x) - b.tau * (-b.alpha1 * (t12 * cpx + t22 * cpy) -
+                                                     b.alpha0 * (qz[j][c] - qzl[c] + qy[j][c] - qyu[c]));
+            }
+            ub[j] = make_float2(2 * un[0] - ou.x, 2 * un[1] - ou.y);
+            vxb[j] = make_float2(2 * xn[0] - ox.x, 2 * xn[1] - ox.y);
+            vyb[j] = make_float2(2 * yn[0] - oy.x, 2 * yn[1] - oy.y);
+            fr[4 * plane] = make_float2(un[0], un[1]);
+            fr[5 * plane] = make_float2(xn[0], xn[1]);
+            fr[6 * plane] = make_float2(yn[0], yn[1]);
+        };
+        auto pair = [](const float (&a)[2]) { return make_float2(a[0], a[1]); };
+#pragma unroll
+        for (int j = 0; j + 1 < RPT; ++j) pq_row(j, ub[j + 1], vxb[j + 1], vyb[j + 1]);
+        __syncthreads();
+        pq_row(RPT - 1, top(0, warp + 1), top(1, warp + 1), top(2, warp + 1));
+        bot(0, warp + 1) = pair(px[RPT - 1]);
+        bot(1, warp + 1) = pair(py[RPT - 1]);
+        bot(2, warp + 1) = pair(qy[RPT - 1]);
+        bot(3, warp + 1) = pair(qz[RPT - 1]);
+#pragma unroll
+        for (int j = RPT - 1; j > 0; --j) u_row(j, pair(px[j - 1]), pair(py[j - 1]), pair(qy[j - 1]), pair(qz[j - 1]));
+        __syncthreads();
+        u_row(0, bot(0, warp), bot(1, warp), bot(2, warp), bot(3, warp));
+    }
+    const int xl = 2 * lane, yl = RPT * warp;
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) {
+        const float2 *fr = sF + (RPT * warp + j) * 32 + lane;
+        const float2 fu = fr[4 * plane], fx = fr[5 * plane], fy = fr[6 * plane];
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            if (in[j][c] && xl + c >= K && xl + c < BW - K && yl + j >= K && yl + j < rows - K) {
+                const size_t i = (size_t)(y0 + j) * w + (xa + c);
+                b.u_out[i] = c ? fu.y : fu.x;
+                b.u1x_out[i] = c ? fx.y : fx.x;
+                b.u1y_out[i] = c ? fy.y : fy.x;
+                b.ubar_out[i] = c ? ub[j].y : ub[j].x;
+                b.u1xbar_out[i] = c ? vxb[j].y : vxb[j].x;
+                b.u1ybar_out[i] = c ? vyb[j].y : vyb[j].x;
+                b.Px_out[i] = px[j][c];
+                b.Py_out[i] = py[j][c];
+                b.Qx_out[i] = qx[j][c];
+                b.Qy_out[i] = qy[j][c];
+                b.Qz_out[i] = qz[j][c];
+                float4 *r4 = reinterpret_cast<float4 *>(b.r_out + i * VS);
+#pragma unroll
+                for (int q = 0; q < VS / 4; ++q) r4[q] = sR[((q * rows + RPT * warp + j) * 2 + c) * 32 + lane];
+            }
+    }
 }
 
 // The energy of the current iterate (the energy checks of the launch path and
@@ -1146,6 +1415,7 @@ struct Layout {
     double *partial, *energy;   // energy_kernel's per-block partial sums (one per tile) and result
     IterCtl *ctl;
     float *exb[2], *exq[2], *exu;
+    float *u2, *u1x2, *u1y2, *r2;   // second buffers of the block form (null where the views' r does not fit)
     double *ppartial;
     unsigned int *bar;
     PersistResult *res;
@@ -1191,6 +1461,12 @@ Layout layout(void *base, int w, int h, int V)
         L.exq[k] = take(5 * n);
     }
     L.exu = take(3 * n);
+    // The block form's second u, v and r lie in the persistent form's exchange
+    // arrays (3 n, then 5 n + 3 n + 5 n + 3 n floats), which it does not use.
+    L.u2 = L.exb[0];
+    L.u1x2 = L.u2 + n;
+    L.u1y2 = L.u1x2 + n;
+    L.r2 = view_stride(V) <= 16 ? L.exq[0] : nullptr;
     L.ppartial = (double *)take(2 * 1024);
     L.bar = (unsigned int *)take(64);
     L.res = (PersistResult *)take(16);
@@ -1615,6 +1891,15 @@ cudaError_t launch_iteration(int V, dim3 grid, dim3 block, cudaStream_t st, cons
     return launch_dependent(iteration_kernel<32>, grid, block, 0, st, ib);
 }
 
+// The block form's kernel for V views (16 at most).
+auto block_kernel(int V)
+{
+    return V <= 4    ? tgv2_block_kernel<4>
+           : V <= 8  ? tgv2_block_kernel<8>
+           : V <= 12 ? tgv2_block_kernel<12>
+                     : tgv2_block_kernel<16>;
+}
+
 int tgv2_run(int w, int h, int V, const float *ref255, const float *srcs255, const float *K9, const float *invK9,
              const float *Rrel, const float *trel, const mvs_tgv2_params *prm, int u_from_input, float u_init,
              float *u, int *iters_out, double *energy_out, void *ws, cudaStream_t st, const TGV2Warm *warm)
@@ -1651,7 +1936,7 @@ int tgv2_run(int w, int h, int V, const float *ref255, const float *srcs255, con
     int total = 0;
     double last_e = 0.0;
     int energy_at = -1;   // iteration count at which last_e was evaluated
-    int cur = 0;          // ping-pong buffer holding the current p, q
+    int cur = 0;          // buffer holding the current state
     bool done = false;
     IterBufs ib;
     ib.ctl = prm->tol > 0 ? L.ctl : nullptr;
@@ -1674,6 +1959,51 @@ int tgv2_run(int w, int h, int V, const float *ref255, const float *srcs255, con
     ib.tau = prm->tau;
     ib.sigma = prm->sigma;
     const dim3 gi(ceil_div(w, TX), ceil_div(h, TY)), bi(TX, TY);
+
+    // Several iterations per launch where that is the faster form, a whole number
+    // of launches between two energy checks.  Measured on the B200 (160x120 to
+    // 640x480, 4 to 8 views), a block launch takes about 5 us plus, for every
+    // warp on the busiest SM, 0.13 + 0.015 VS us an iteration (VS views, a
+    // multiple of 4; the loads count as two iterations), and the launch of one
+    // iteration 4 us plus its L2 bytes at 7.9 TB/s.  So the block form takes the
+    // small frames (320x240, 4 views: 100 iterations in 435 us against 577;
+    // 160x120, 5 views: 379 against 458) and leaves the large ones, whose
+    // views' state does not fit on the chip at once, to one launch per iteration
+    // (640x480, 8 views: 1.43 ms against 1.27).
+    const int segment = prm->tol > 0 ? min(check_every, prm->niters) : prm->niters;
+    bool blocked = prm->iteration_kernel == MVS_TGV2_ITER_AUTO && L.r2 && segment > 1;
+    BlockPlan plan{1, 0};
+    size_t bsmem = 0;
+    BlockBufs bb;
+    if (blocked) {
+        const int VS = view_stride(V), fit = (int)((kSmemMax - kBlockBytes) / block_warp_bytes(V));
+        double us = 0.0;
+        plan = block_plan(w, h, segment, min(TGW, fit), 5.0, 0.13 + 0.015 * VS, 2, &us);
+        plan.iters = ceil_div(segment, ceil_div(segment, plan.iters));   // equal shares
+        blocked = us < segment * (4.0 + (double)n * (8 * (8 + V) + 4 * (4 + 2 * V)) / 7.9e6);
+    }
+    if (blocked) {
+        bsmem = block_warp_bytes(V) * plan.warps + kBlockBytes;
+        MVS_TRY_CUDA(cudaFuncSetAttribute(block_kernel(V), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
+        bb.ctl = ib.ctl;
+        bb.T11 = L.T11;
+        bb.T12 = L.T12;
+        bb.T22 = L.T22;
+        bb.u0 = L.u0;
+        bb.It = L.It;
+        bb.Iu = L.Iu;
+        bb.w = w;
+        bb.h = h;
+        bb.V = V;
+        bb.lambda = prm->lambda;
+        bb.alpha0 = prm->alpha0;
+        bb.alpha1 = prm->alpha1;
+        bb.tau = prm->tau;
+        bb.sigma = prm->sigma;
+    }
+    // u, v and r: two buffers in the block form, updated in place otherwise
+    float *const U[2] = {u, blocked ? L.u2 : u}, *const U1X[2] = {L.u1x, blocked ? L.u1x2 : L.u1x};
+    float *const U1Y[2] = {L.u1y, blocked ? L.u1y2 : L.u1y}, *const RV[2] = {L.r, blocked ? L.r2 : L.r};
 
     // on-chip persistent iterations when the image fits one tile per SM
     int pth = 0, ptiles = 0;
@@ -1722,24 +2052,25 @@ int tgv2_run(int w, int h, int V, const float *ref255, const float *srcs255, con
         if (!pth && prm->tol > 0 && l > 0)   // a new linearisation has no previous energy
             MVS_TRY_CUDA(cudaMemsetAsync(&L.ctl->n_hist, 0, sizeof(int), st));
         if (warm && l == 0)
-            warm_init_kernel<<<eg, 256, 0, st>>>(n, V, warm->u_lin, u, warm->v, warm->v ? warm->v + n : nullptr, L.u0,
-                                                L.ubar[0], L.u1x, L.u1y, L.u1xbar[0], L.u1ybar[0], L.Px[0], L.Py[0],
-                                                L.Qx[0], L.Qy[0], L.Qz[0], L.r, warm->pq, warm->r);
+            warm_init_kernel<<<eg, 256, 0, st>>>(n, V, warm->u_lin, U[cur], warm->v, warm->v ? warm->v + n : nullptr,
+                                                L.u0, L.ubar[cur], U1X[cur], U1Y[cur], L.u1xbar[cur], L.u1ybar[cur],
+                                                L.Px[cur], L.Py[cur], L.Qx[cur], L.Qy[cur], L.Qz[cur], RV[cur],
+                                                warm->pq, warm->r);
         else
-            warp_init_kernel<<<eg, 256, 0, st>>>(n, V, u, L.u0, L.ubar[0], L.u1x, L.u1y, L.u1xbar[0], L.u1ybar[0],
-                                                L.Px[0], L.Py[0], L.Qx[0], L.Qy[0], L.Qz[0], L.r);
+            warp_init_kernel<<<eg, 256, 0, st>>>(n, V, U[cur], L.u0, L.ubar[cur], U1X[cur], U1Y[cur], L.u1xbar[cur],
+                                                L.u1ybar[cur], L.Px[cur], L.Py[cur], L.Qx[cur], L.Qy[cur], L.Qz[cur],
+                                                RV[cur]);
         linearize_kernel<<<dim3(g2.x, g2.y, V), b2, 0, st>>>(cams, srcs255, L.ref01, L.u0, w, h, L.It, L.Iu);
         if (warm && l == 0) {
             const int do_pq = !warm->pq && warm->dual_sigma > 0, do_r = !warm->r && warm->dual_sigma_r > 0;
             if (do_pq || do_r)
-                dual_init_kernel<<<g2, b2, 0, st>>>(L.T11, L.T12, L.T22, L.It, L.Iu, L.u0, u, L.u1x, L.u1y, w, h, V,
-                                                   prm->lambda, prm->alpha0, prm->alpha1, (float)warm->dual_sigma,
-                                                   (float)warm->dual_sigma_r, L.Px[0], L.Py[0], L.Qx[0], L.Qy[0],
-                                                   L.Qz[0], L.r, do_pq, do_r);
+                dual_init_kernel<<<g2, b2, 0, st>>>(L.T11, L.T12, L.T22, L.It, L.Iu, L.u0, U[cur], U1X[cur], U1Y[cur], w,
+                                                   h, V, prm->lambda, prm->alpha0, prm->alpha1,
+                                                   (float)warm->dual_sigma, (float)warm->dual_sigma_r, L.Px[cur],
+                                                   L.Py[cur], L.Qx[cur], L.Qy[cur], L.Qz[cur], RV[cur], do_pq, do_r);
         }
         rc = check_launch("tgv2 linearisation");
         if (rc) break;
-        cur = 0;
         if (pth) {
             // the whole linearisation in one cooperative launch
             PersistBufs pb;
@@ -1810,33 +2141,69 @@ int tgv2_run(int w, int h, int V, const float *ref255, const float *srcs255, con
             done = hr.done || total >= cap;
             continue;
         }
-        const int warp_start = launched;
-        for (int k = 0; k < prm->niters; ++k) {
-            ib.ubar_in = L.ubar[cur];
-            ib.u1xbar_in = L.u1xbar[cur];
-            ib.u1ybar_in = L.u1ybar[cur];
-            ib.Px_in = L.Px[cur];
-            ib.Py_in = L.Py[cur];
-            ib.Qx_in = L.Qx[cur];
-            ib.Qy_in = L.Qy[cur];
-            ib.Qz_in = L.Qz[cur];
-            ib.ubar_out = L.ubar[cur ^ 1];
-            ib.u1xbar_out = L.u1xbar[cur ^ 1];
-            ib.u1ybar_out = L.u1ybar[cur ^ 1];
-            ib.Px_out = L.Px[cur ^ 1];
-            ib.Py_out = L.Py[cur ^ 1];
-            ib.Qx_out = L.Qx[cur ^ 1];
-            ib.Qy_out = L.Qy[cur ^ 1];
-            ib.Qz_out = L.Qz[cur ^ 1];
-            // dependent launches: each iteration's launch overlaps the previous one's tail
-            MVS_TRY_CUDA(launch_iteration(V, gi, bi, st, ib));
-            cur ^= 1;
-            ++launched;
-            const bool check = prm->tol > 0 && (k + 1) % check_every == 0;
+        const int warp_start = launched, cur_start = cur;
+        for (int k = 0; k < prm->niters;) {
+            const int nxt = cur ^ 1;
+            int steps = 1;
+            if (blocked) {
+                steps = min(plan.iters, min(segment - k % segment, min(prm->niters - k, max(cap - launched, 1))));
+                bb.iters = steps;
+                bb.halo = block_halo(steps);
+                bb.first = k == 0;
+                bb.u_in = U[cur];
+                bb.u1x_in = U1X[cur];
+                bb.u1y_in = U1Y[cur];
+                bb.r_in = RV[cur];
+                bb.ubar_in = L.ubar[cur];
+                bb.u1xbar_in = L.u1xbar[cur];
+                bb.u1ybar_in = L.u1ybar[cur];
+                bb.Px_in = L.Px[cur];
+                bb.Py_in = L.Py[cur];
+                bb.Qx_in = L.Qx[cur];
+                bb.Qy_in = L.Qy[cur];
+                bb.Qz_in = L.Qz[cur];
+                bb.u_out = U[nxt];
+                bb.u1x_out = U1X[nxt];
+                bb.u1y_out = U1Y[nxt];
+                bb.r_out = RV[nxt];
+                bb.ubar_out = L.ubar[nxt];
+                bb.u1xbar_out = L.u1xbar[nxt];
+                bb.u1ybar_out = L.u1ybar[nxt];
+                bb.Px_out = L.Px[nxt];
+                bb.Py_out = L.Py[nxt];
+                bb.Qx_out = L.Qx[nxt];
+                bb.Qy_out = L.Qy[nxt];
+                bb.Qz_out = L.Qz[nxt];
+                MVS_TRY_CUDA(launch_dependent(block_kernel(V), block_grid(w, h, steps, plan.warps),
+                                              dim3(32 * plan.warps), bsmem, st, bb));
+            } else {
+                ib.ubar_in = L.ubar[cur];
+                ib.u1xbar_in = L.u1xbar[cur];
+                ib.u1ybar_in = L.u1ybar[cur];
+                ib.Px_in = L.Px[cur];
+                ib.Py_in = L.Py[cur];
+                ib.Qx_in = L.Qx[cur];
+                ib.Qy_in = L.Qy[cur];
+                ib.Qz_in = L.Qz[cur];
+                ib.ubar_out = L.ubar[nxt];
+                ib.u1xbar_out = L.u1xbar[nxt];
+                ib.u1ybar_out = L.u1ybar[nxt];
+                ib.Px_out = L.Px[nxt];
+                ib.Py_out = L.Py[nxt];
+                ib.Qx_out = L.Qx[nxt];
+                ib.Qy_out = L.Qy[nxt];
+                ib.Qz_out = L.Qz[nxt];
+                // dependent launches: each iteration's launch overlaps the previous one's tail
+                MVS_TRY_CUDA(launch_iteration(V, gi, bi, st, ib));
+            }
+            cur = nxt;
+            k += steps;
+            launched += steps;
+            const bool check = prm->tol > 0 && k % check_every == 0;
             if (check)
-                MVS_TRY_CUDA(launch_dependent(energy_kernel, gi, bi, 0, st, L.T11, L.T12, L.T22, L.It, L.Iu, L.u0, u,
-                                              L.u1x, L.u1y, w, h, V, prm->lambda, prm->alpha0, prm->alpha1, L.partial,
-                                              L.energy, L.ctl, prm->tol, launched, stop_window));
+                MVS_TRY_CUDA(launch_dependent(energy_kernel, gi, bi, 0, st, L.T11, L.T12, L.T22, L.It, L.Iu, L.u0, U[cur],
+                                              U1X[cur], U1Y[cur], w, h, V, prm->lambda, prm->alpha0, prm->alpha1,
+                                              L.partial, L.energy, L.ctl, prm->tol, launched, stop_window));
             if (launched >= cap) {
                 done = true;
                 break;
@@ -1847,7 +2214,7 @@ int tgv2_run(int w, int h, int V, const float *ref255, const float *srcs255, con
                 if (e == cudaSuccess) e = sp.due(launched, &L.ctl->done, &hc.done, &read);
                 if (e != cudaSuccess) sp.fail();
                 else if (read && hc.done) break;
-            } else if (prm->tol > 0 && launched % kPoll == 0) {
+            } else if (prm->tol > 0 && (launched - warp_start) / kPoll != (launched - steps - warp_start) / kPoll) {
                 if ((rc = poll())) break;
                 if (hc.done) break;
             }
@@ -1857,7 +2224,11 @@ int tgv2_run(int w, int h, int V, const float *ref255, const float *srcs255, con
             rc = poll();
             if (!rc && hc.done) {
                 done = true;
-                cur = (hc.stop_total - warp_start) & 1;   // p, q of the last iteration that ran
+                // the buffers of the last launch that ran: a stop falls on a check, so
+                // after a whole number of segments
+                const int ran = hc.stop_total - warp_start;
+                const int launches = blocked ? ran / segment * ceil_div(segment, plan.iters) : ran;
+                cur = cur_start ^ (launches & 1);
             }
         }
         if (!rc) rc = check_launch("tgv2 iteration");
@@ -1871,9 +2242,13 @@ int tgv2_run(int w, int h, int V, const float *ref255, const float *srcs255, con
             energy_at = hc.energy_at;
         }
     }
+    if (!rc && U[cur] != u) {   // the result in the caller's buffer
+        cudaMemcpyAsync(u, U[cur], n * sizeof(float), cudaMemcpyDeviceToDevice, st);
+        rc = check_launch("tgv2 u readout");
+    }
     if (!rc && warm && warm->v) {
-        cudaMemcpyAsync(warm->v, L.u1x, n * sizeof(float), cudaMemcpyDeviceToDevice, st);
-        cudaMemcpyAsync(warm->v + n, L.u1y, n * sizeof(float), cudaMemcpyDeviceToDevice, st);
+        cudaMemcpyAsync(warm->v, U1X[cur], n * sizeof(float), cudaMemcpyDeviceToDevice, st);
+        cudaMemcpyAsync(warm->v + n, U1Y[cur], n * sizeof(float), cudaMemcpyDeviceToDevice, st);
         rc = check_launch("tgv2 v readout");
     }
     if (!rc && warm && warm->pq) {
@@ -1883,13 +2258,13 @@ int tgv2_run(int w, int h, int V, const float *ref255, const float *srcs255, con
         rc = check_launch("tgv2 dual readout");
     }
     if (!rc && warm && warm->r) {   // the caller's [V][n] planes
-        r_planes_kernel<<<eg, 256, 0, st>>>(L.r, n, V, warm->r);
+        r_planes_kernel<<<eg, 256, 0, st>>>(RV[cur], n, V, warm->r);
         rc = check_launch("tgv2 dual readout");
     }
     if (!rc && energy_out && energy_at != total) {
         // energy of the final iterate for callers that ask for it
-        energy_kernel<<<gi, bi, 0, st>>>(L.T11, L.T12, L.T22, L.It, L.Iu, L.u0, u, L.u1x, L.u1y, w, h, V, prm->lambda,
-                                         prm->alpha0, prm->alpha1, L.partial, L.energy, L.ctl, 0.0, total, 1);
+        energy_kernel<<<gi, bi, 0, st>>>(L.T11, L.T12, L.T22, L.It, L.Iu, L.u0, U[cur], U1X[cur], U1Y[cur], w, h, V,
+                                         prm->lambda, prm->alpha0, prm->alpha1, L.partial, L.energy, L.ctl, 0.0, total, 1);
         cudaMemcpyAsync(h_energy, L.energy, sizeof(double), cudaMemcpyDeviceToHost, st);
         cudaError_t e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) rc = set_error(MVS_ERR_CUDA, "tgv2 energy: %s", cudaGetErrorString(e));
