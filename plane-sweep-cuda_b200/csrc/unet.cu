@@ -719,26 +719,44 @@ __global__ void __launch_bounds__(WG_THREADS) wgrad_kernel(const bf16 *__restric
     }
 }
 
-// bias gradient: db[co] += sum_p dz[p][co]
-__global__ void bgrad_kernel(const bf16 *__restrict__ dz, long long npix, int cout, int px_per_cta,
-                             float *__restrict__ db)
+// bias gradient: db[co] += sum_p dz[p][co].  HBM-bound: a thread sums 16-byte
+// groups of 8 channels of every `rows`-th pixel of its block's run, four loads
+// in flight; runs are sized for four blocks per SM (at least 256 pixels).
+// Against one channel per thread and 2048 pixels per block (cold caches, B200):
+// 640x480 x 4, 16 channels, 22 -> 11 us; 80x60 x 4, 128 channels, which gave
+// only 10 blocks, 134 -> 8 us.
+__global__ void __launch_bounds__(256) bgrad_kernel(const bf16 *__restrict__ dz, long long npix, int cout,
+                                                    int px_per_cta, float *__restrict__ db)
 {
-    __shared__ float red[256];
-    const int tid = threadIdx.x;
-    const int lanes = 256 / cout * cout;   // threads used: a multiple of cout
-    float s = 0.f;
-    if (tid < lanes) {
-        const int co = tid % cout, row = tid / cout, rows = lanes / cout;
-        const long long p0 = (long long)blockIdx.x * px_per_cta;
-        const long long p1 = min(p0 + px_per_cta, npix);
-        for (long long p = p0 + row; p < p1; p += rows) s += bf2f(dz[(size_t)p * cout + co]);
-    }
-    red[tid] = s;
-    __syncthreads();
-    if (tid < cout) {
-        float t = 0.f;
-        for (int k = tid; k < lanes; k += cout) t += red[k];
-        atomicAdd(&db[tid], t);
+    __shared__ float red[256][9];   // 9: no bank conflicts
+    const int tid = threadIdx.x, groups = cout >> 3;
+    const long long p0 = (long long)blockIdx.x * px_per_cta, p1 = min(p0 + px_per_cta, npix);
+    for (int g0 = 0; g0 < groups; g0 += 256) {   // one pass up to 2048 channels
+        const int gn = min(groups - g0, 256), rows = 256 / gn;
+        const int g = tid % gn, row = tid / gn;
+        float s[8] = {};
+        if (row < rows) {
+            const uint4 *q = (const uint4 *)dz + g0 + g;
+#pragma unroll 4
+            for (long long p = p0 + row; p < p1; p += rows) {
+                const uint4 v = __ldg(q + (size_t)p * groups);
+                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    s[2 * k] += bf2f((uint16_t)(w[k] & 0xffffu));
+                    s[2 * k + 1] += bf2f((uint16_t)(w[k] >> 16));
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 8; ++k) red[tid][k] = s[k];
+        __syncthreads();
+        for (int c = tid; c < 8 * gn; c += 256) {
+            float t = 0.f;
+            for (int r = 0; r < rows; ++r) t += red[r * gn + (c >> 3)][c & 7];
+            atomicAdd(&db[8 * g0 + c], t);
+        }
     }
 }
 
@@ -754,7 +772,10 @@ int launch_wgrad(const bf16 *x, int cin, const bf16 *dz, int cout, int B, int H,
     } else {
         MVS_RC_(launch_wgrad_cuda_cores(x, cin, dz, cout, B, H, W, dW, st));
     }
-    if (db) bgrad_kernel<<<(int)((npix + 2047) / 2048), 256, 0, st>>>(dz, npix, cout, 2048, db);
+    if (db) {
+        const int px = (int)std::max<long long>(256, (npix + 4 * kSMs - 1) / (4 * kSMs));
+        bgrad_kernel<<<(int)((npix + px - 1) / px), 256, 0, st>>>(dz, npix, cout, px, db);
+    }
     return MVS_OK;
 }
 
