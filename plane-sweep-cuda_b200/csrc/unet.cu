@@ -337,20 +337,17 @@ int launch_conv(const bf16 *in, int cin, const bf16 *wpack, const float *bias, c
 }
 
 // ---------------------------------------------------------------------------
-// weight gradient on tensor cores: for every tap t = (ky, kx),
-//   D[co][t][ci] += sum_p dz[p][co] * x[p + off_t][ci]
-// with K = pixels, for 16-channel chunks of the input.  A = dz^T (M = co, up
-// to 128 rows) and B = the nine tap-shifted copies of the input tile (N = 9
-// taps x 16 channels = 144) are both MN-major with the same layout,
-// [8-group][pixel][8]: A as [co/8][pixel][8], B as [tap][ci/8][pixel][8] where
-// plane (t, g) holds x at the tile's pixels shifted by tap t's offset.  One K
-// step of 16 pixels (two tile rows) is then a single MMA for all nine taps (8
-// per tile, with N = 144), instead of one MMA per tap (72 with N = 16).  A CTA
-// takes NCH = 1 or 2 chunks (16 or 32 input channels) against one staged dz
-// tile: NCH MMAs per K step into NCH accumulators.  The tap planes are built
-// in shared memory from the tile's input halo (wgrad_tc_kernel below); each
-// CTA sums a run of pixel tiles in TMEM (144 NCH columns) and adds them to the
-// FP32 gradient with one atomic per weight.
+// weight gradient on tensor cores: for every tap (ky, kx),
+//   D[co][kx][ky][ci] += sum_p dz[p][co] * x[p + (ky, kx)][ci]
+// with K = pixels, for 16-channel chunks of the input.  A = dz^T (M = 64 or 128
+// output channels) is MN-major, [co / 8][pixel][8].  B is the tile's input halo
+// itself, stored so that one descriptor reaches three taps: rows of 10 pixels x
+// 16 bytes ordered [halo row][8-channel group], so the (ky, group) neighbour of
+// a core matrix (8 pixels of a tile row x 8 channels) lies 160 bytes further
+// for each step of 2 ky + group, the next tile row 320 bytes further, and tap
+// kx starts 16 kx bytes later.  A K-step of 16 pixels (two tile rows) is then
+// three MMAs with N = 3 ky x 16 channels = 48, straight from the bytes that
+// cp.async brought: nothing is expanded or copied in shared memory.
 // ---------------------------------------------------------------------------
 
 struct WgArgs {
@@ -359,40 +356,33 @@ struct WgArgs {
     float *dW;        // [cout][cin][9]
     int *err;
     int B, H, W, cin, cout, tiles_x, tiles_y, tiles_per_cta, n_tiles;
-    int ci_base;      // first input channel of blockIdx.y == 0
+    int vec;          // dW is 16-byte aligned
 };
 
 constexpr int WG_TC_THREADS = 256;
-constexpr int WG_NC = 16;                           // input channels per chunk
-constexpr int WG_PLANES = 9 * WG_NC / 8;            // 18 B planes per chunk: (tap, channel group)
-
-// Shared memory of wgrad_tc_kernel<NCH, R> for `cg` groups of 8 output
-// channels (cg <= 16):
-//   two MMA buffers, each A = dz [cg][128 pixels][16 B] followed by, per
-//     16-channel chunk, B = the nine tap-shifted input planes
-//     [tap][channel group][128 pixels][16 B] (18 planes);
-//   R raw stages, each the dz tile [cg][128][16 B] and, per chunk, the input
-//     halo [channel group][18 rows][10 columns][16 B], filled by cp.async.
-// The A descriptor of an M = 128 MMA spans 16 groups (32 KB) from A's start;
-// groups past cg read the B planes that follow and only fill accumulator rows
-// co >= cout, which are never stored, so A needs no zero padding.
+constexpr int WG_NC = 16;                                      // input channels per chunk
 constexpr int WG_HALO_W = TW + 2, WG_HALO_H = TH + 2;          // 10 x 18 input pixels around an 8 x 16 tile
-constexpr int WG_HALO_BYTES = 2 * WG_HALO_H * WG_HALO_W * 16;  // per chunk: 5760
-constexpr int WG_PLANES_BYTES = WG_PLANES * 128 * 16;          // per chunk: 36864
-constexpr int WG_SMEM_MAX = 227 * 1024;
+constexpr int WG_HALO_BYTES = 2 * WG_HALO_H * WG_HALO_W * 16;  // 5760
+constexpr int WG_N = 3 * WG_NC;                                // columns of one MMA: (ky, channel)
 constexpr int WG_SMEM_SM = 228 * 1024;   // shared memory of an SM, 1 KB of it reserved per CTA
+constexpr int WG_MAX_STAGES = 8;
+// tiles a CTA sums at least: each adds its 9 x 16 x cout sums to dW atomically
+constexpr int WG_MIN_TILES = 8;
 
+// Shared memory for `cg` groups of 8 output channels: `stages` x (dz tile [cg]
+// [128 pixels][16 B], input halo), then room for what an A descriptor of M rows
+// spans past the last stage's groups.  (The groups past cg read other bytes of
+// the ring and only fill accumulator rows co >= cout, which are never stored.)
 struct WgLayout {
-    int a_bytes, buf_bytes, raw_bytes, bytes;
+    int a_bytes, stage_bytes, bytes;
 };
 
-__host__ __device__ inline WgLayout wg_layout(int nch, int stages, int cg)
+__host__ __device__ inline WgLayout wg_layout(int m, int stages, int cg)
 {
     WgLayout L;
     L.a_bytes = cg * 128 * 16;
-    L.buf_bytes = L.a_bytes + nch * WG_PLANES_BYTES;
-    L.raw_bytes = L.a_bytes + nch * WG_HALO_BYTES;
-    L.bytes = 2 * L.buf_bytes + stages * L.raw_bytes + 64;
+    L.stage_bytes = L.a_bytes + WG_HALO_BYTES;
+    L.bytes = stages * L.stage_bytes + (m / 8) * 128 * 16 + 128;
     return L;
 }
 
@@ -403,36 +393,52 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// The weight gradient of a 3x3 convolution on the tensor cores:
-// dW[co][ci][tap] = sum over pixels of dz[co][p] x[ci][p + tap], K = pixels.
-// Per 8 x 16 tile: the raw stage lands (cp.async, R - 1 tiles ahead), the CTA
-// copies its dz tile and expands its input halo into the nine tap-shifted
-// planes of an MMA buffer (shared-memory loads and stores: the input crosses
-// L2 once instead of nine times), and one thread issues 8 K-steps of one
-// MMA of 128 x (9 taps x 16 channels) x 16 pixels per chunk.  The two MMA
-// buffers alternate; a buffer is rebuilt once the MMAs that read it have
-// signalled its mbarrier (tcgen05.commit).  Every wait is bounded.
-template <int NCH, int R>
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4])
+{
+    uint32_t r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = __uint_as_float(r[k]);
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void red_add4(float *dst, float a, float b, float c, float d)
+{
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+// A CTA sums a run of 8 x 16 tiles for one 16-channel chunk of the input
+// (blockIdx.y) and one block of M output channels (blockIdx.z) in tensor memory:
+// a ring of R stages is filled by cp.async R - 1 tiles ahead, one thread issues
+// the 24 MMAs of a tile, and tcgen05.commit on the stage's mbarrier frees it.
+// Every wait is bounded.  M = 64 keeps rows 16 q .. 16 q + 15 of the accumulator
+// in lanes 32 q .. 32 q + 15.
+//
+// What bounds it: shared-memory reads of the MMAs (3.5 KB each at M = 64, 24 per
+// tile and chunk) and, on the inner levels, the latency of few tiles per CTA.
+template <int M, int R>
 __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
 {
-    static_assert(R >= 2, "at least two raw stages");
-    constexpr int NBUF = 2;   // MMA buffers
+    static_assert(R >= 2 && R <= WG_MAX_STAGES, "at least two stages");
+    constexpr int TMEM_COLS = 256;   // 3 WG_N = 144 used
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ci0 = a.ci_base + blockIdx.y * NCH * WG_NC, co0 = blockIdx.z * 128;
-    const int cg = min(a.cout - co0, 128) >> 3;
-    const WgLayout L = wg_layout(NCH, R, cg);
-    uint64_t *bars = (uint64_t *)(smem + NBUF * L.buf_bytes + R * L.raw_bytes);
-    uint32_t *tmem_slot = (uint32_t *)(smem + NBUF * L.buf_bytes + R * L.raw_bytes + 32);
+    const int ci0 = blockIdx.y * WG_NC, co0 = blockIdx.z * M;
+    const int cg = min(a.cout - co0, M) >> 3;
+    const WgLayout L = wg_layout(M, R, cg);
+    uint64_t *bars = (uint64_t *)(smem + L.bytes - 128);
+    uint32_t *tmem_slot = (uint32_t *)(smem + L.bytes - 128 + 8 * WG_MAX_STAGES);
     const int t_begin = blockIdx.x * a.tiles_per_cta;
     const int t_end = min(t_begin + a.tiles_per_cta, a.n_tiles);
     const int H = a.H, W = a.W, cin = a.cin, cout = a.cout;
     const size_t img = (size_t)H * W;
-    constexpr int TMEM_COLS = NCH == 1 ? 256 : 512;   // 144 NCH used
 
     if (warp == 0) tmem_alloc(tmem_slot, TMEM_COLS);
     if (tid == 0) {
-        for (int k = 0; k < NBUF; ++k) mbar_init(&bars[k], 1);
+        for (int k = 0; k < R; ++k) mbar_init(&bars[k], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     tc_fence_before();
@@ -440,30 +446,28 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t sbase = smem_u32(smem);
-    const uint32_t rbase = sbase + NBUF * L.buf_bytes;
 
     // Each thread's copies are the same for every tile: dz pixel (tid & 127) of
-    // the groups tid >> 7, + 2, ...; halo items tid, tid + 256, ... (chunk and
-    // channel group, halo row, halo column), worked out once here.
-    constexpr int HP = WG_HALO_H * WG_HALO_W;
-    constexpr int HALO_ITEMS = NCH * 2 * HP;
+    // the groups tid >> 7, + 2, ...; halo items tid, tid + 256 (halo pixel,
+    // then channel group), worked out once here.
+    constexpr int HALO_ITEMS = 2 * WG_HALO_H * WG_HALO_W;
     constexpr int HI = (HALO_ITEMS + WG_TC_THREADS - 1) / WG_TC_THREADS;
     const int dz_m = tid & 127, dz_y = dz_m >> 3, dz_x = dz_m & 7, dz_g0 = tid >> 7;
-    int h_jg[HI], h_y[HI], h_x[HI];
+    int h_y[HI], h_x[HI], h_dst[HI];
 #pragma unroll
     for (int i = 0; i < HI; ++i) {
         const int k = tid + i * WG_TC_THREADS;
-        const int jg = k / HP, pix = k - jg * HP;
-        h_jg[i] = k < HALO_ITEMS ? jg : -1;
-        h_y[i] = pix / WG_HALO_W - 1;
-        h_x[i] = pix - (pix / WG_HALO_W) * WG_HALO_W - 1;
+        const int pix = k >> 1, g = k & 1, y = pix / WG_HALO_W, x = pix - y * WG_HALO_W;
+        h_y[i] = y - 1;
+        h_x[i] = x - 1;
+        h_dst[i] = k < HALO_ITEMS ? ((y * 2 + g) * WG_HALO_W + x) * 16 : -1;
     }
-    // cp.async of tile `tile`'s dz and input halo into raw stage s (one commit group)
+    const bf16 *xg = a.x + ci0 + 8 * (tid & 1);
+    // cp.async of tile `tile`'s dz and input halo into stage s (one commit group)
     auto load = [&](int tile, int s) {
         const int b = tile / (a.tiles_x * a.tiles_y), r = tile - b * a.tiles_x * a.tiles_y;
         const int y0 = (r / a.tiles_x) * TH, x0 = (r % a.tiles_x) * TW;
-        const uint32_t ab = rbase + s * L.raw_bytes, hb = ab + L.a_bytes;
-        const bf16 *xb = a.x + (size_t)b * img * cin + ci0;
+        const uint32_t ab = sbase + s * L.stage_bytes, hb = ab + L.a_bytes;
         {
             const int gy = y0 + dz_y, gx = x0 + dz_x;
             const bool ok = gy < H && gx < W;
@@ -472,38 +476,15 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
         }
 #pragma unroll
         for (int i = 0; i < HI; ++i) {
-            if (h_jg[i] < 0) continue;
+            if (h_dst[i] < 0) continue;
             const int gy = y0 + h_y[i], gx = x0 + h_x[i];
             const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
-            const bf16 *src = xb + (ok ? (size_t)gy * W + gx : 0) * cin + 8 * h_jg[i];
-            cp_async16(hb + (tid + i * WG_TC_THREADS) * 16, src, ok);
+            cp_async16(hb + h_dst[i], xg + ((size_t)b * img + (ok ? (size_t)gy * W + gx : 0)) * cin, ok);
         }
         cp_async_commit();
     };
-    // raw stage s -> MMA buffer q: the dz tile as is, the halo as nine
-    // tap-shifted planes (thread = tile pixel m and one of the two channel
-    // groups of each chunk, 16 B per plane)
-    auto build = [&](int s, int q) {
-        const uint4 *ra = (const uint4 *)(smem + NBUF * L.buf_bytes + s * L.raw_bytes);
-        const uint4 *rh = ra + L.a_bytes / 16;
-        uint4 *ba = (uint4 *)(smem + q * L.buf_bytes);
-        uint4 *bp = ba + L.a_bytes / 16;
-        for (int k = tid; k < cg * 128; k += WG_TC_THREADS) ba[k] = ra[k];
-        const int m = tid & 127, my = m >> 3, mx = m & 7, g = tid >> 7;
-#pragma unroll
-        for (int j = 0; j < NCH; ++j) {
-            const int jg = 2 * j + g;
-            const uint4 *h = rh + jg * WG_HALO_H * WG_HALO_W;
-            uint4 *dst = bp + j * (WG_PLANES_BYTES / 16) + g * 128 + m;
-#pragma unroll
-            for (int t = 0; t < 9; ++t) {
-                const int ky = t / 3, kx = t - 3 * ky;
-                dst[t * 2 * 128] = h[(my + ky) * WG_HALO_W + mx + kx];
-            }
-        }
-    };
 
-    constexpr uint32_t idesc = idesc_bf16_mn(128, 9 * WG_NC);
+    constexpr uint32_t idesc = idesc_bf16_mn(M, WG_N);
     const int n = t_end - t_begin;
     bool failed = false;
     int last = -1;   // the last tile whose MMAs were issued (the same in every thread)
@@ -511,46 +492,46 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
         if (k < n) load(t_begin + k, k);
         else cp_async_commit();   // empty groups keep the group count per tile fixed
     }
-    // tile c's MMAs read buffer c % NBUF and signal bars[c % NBUF]; that is the
-    // barrier's (c / NBUF)-th completion, of parity (c / NBUF) & 1
+    // tile c's MMAs read stage c % R and signal bars[c % R]: that barrier's
+    // (c / R)-th completion, of parity (c / R) & 1
     for (int c = 0; c < n; ++c) {
-        const int q = c % NBUF;
         cp_async_wait_group<R - 2>();   // tile c's group landed (R - 2 newer ones may be in flight)
-        // the MMAs of tile c - NBUF read buffer q
-        const bool ok = c < NBUF || mbar_wait_bounded(&bars[q], (uint32_t)(((c - NBUF) / NBUF) & 1), kWaitNs);
-        // every thread's copies of tile c landed, buffer q is free, raw stage (c - 1) % R is free
-        failed = __syncthreads_or(!ok) != 0;
+        fence_async_smem();             // visible to the MMAs
+        failed = __syncthreads_or(failed) != 0;
         if (failed) break;
-        if (c + R - 1 < n) load(t_begin + c + R - 1, (c + R - 1) % R);
-        else cp_async_commit();
-        build(c % R, q);
-        fence_async_smem();   // the generic-proxy stores, visible to the MMAs
-        __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            const uint32_t ab = sbase + q * L.buf_bytes, bb = ab + L.a_bytes;
+            const uint32_t ab = sbase + (c % R) * L.stage_bytes, hb = ab + L.a_bytes;
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks) {
                 const uint64_t ad = smem_desc(ab + ks * 256, 128, 128 * 16);
 #pragma unroll
-                for (int j = 0; j < NCH; ++j) {
-                    const uint64_t bd = smem_desc(bb + j * WG_PLANES_BYTES + ks * 256, 128, 128 * 16);
-                    mma_bf16(tmem + j * 9 * WG_NC, ad, bd, idesc, (c > 0 || ks > 0) ? 1u : 0u);
+                for (int kx = 0; kx < 3; ++kx) {
+                    const uint64_t bd = smem_desc(hb + (4 * ks * WG_HALO_W + kx) * 16, 2 * WG_HALO_W * 16, WG_HALO_W * 16);
+                    mma_bf16(tmem + kx * WG_N, ad, bd, idesc, (c > 0 || ks > 0) ? 1u : 0u);
                 }
             }
-            mma_commit(&bars[q]);
+            mma_commit(&bars[c % R]);
         }
         last = c;
+        if (c + R - 1 < n) {
+            // stage (c - 1) % R takes tile c + R - 1 once tile c - 1's MMAs have read it
+            failed = c >= 1 && !mbar_wait_bounded(&bars[(c - 1) % R], (uint32_t)(((c - 1) / R) & 1), kWaitNs);
+            if (!failed) load(t_begin + c + R - 1, (c + R - 1) % R);
+        } else {
+            cp_async_commit();
+        }
     }
+    failed = __syncthreads_or(failed) != 0;
     if (!failed && last >= 0) {
-        const bool ok = mbar_wait_bounded(&bars[last % NBUF], (uint32_t)((last / NBUF) & 1), kWaitNs);
+        const bool ok = mbar_wait_bounded(&bars[last % R], (uint32_t)((last / R) & 1), kWaitNs);
         failed = __syncthreads_or(!ok) != 0;
     }
+    cp_async_wait_group<0>();
     if (failed) {
         if (tid == 0) atomicExch(a.err, 1);
-        cp_async_wait_group<0>();   // copies in flight
-        if (last >= 0)              // the MMAs in flight (they complete in order)
-            mbar_wait_bounded(&bars[last % NBUF], (uint32_t)((last / NBUF) & 1), kWaitNs);
+        if (last >= 0)   // the MMAs in flight (they complete in order)
+            mbar_wait_bounded(&bars[last % R], (uint32_t)((last / R) & 1), kWaitNs);
         tc_fence_before();
         __syncthreads();
         if (warp == 0) {
@@ -559,22 +540,30 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
         }
         return;
     }
-    cp_async_wait_group<0>();   // the trailing empty groups
     tc_fence_after();
     if (n > 0) {
-        // D[co][n], n = tap * 16 + channel: TMEM lane = co; warps w and w + 4
-        // read lanes 32 (w % 4) .. + 31, the even and the odd (chunk, tap) columns
+        // D[co][kx][ky][ci]; warps w and w + 4 read lanes 32 (w % 4) .. + 31, the
+        // even and the odd groups of four channels: 36 consecutive values of dW
         const int quarter = warp & 3;
-        const int co = co0 + quarter * 32 + lane;
+        const int row = M == 128 ? quarter * 32 + lane : quarter * 16 + lane;
+        const bool own = (M == 128 || lane < 16) && co0 + row < cout;
+        float *dst = a.dW + ((size_t)(co0 + row) * cin + ci0) * 9;
 #pragma unroll 1
-        for (int qq = warp >> 2; qq < 9 * NCH; qq += 2) {   // (chunk, tap)
-            const int j = qq / 9, t = qq - 9 * j;
-            float v[16];
-            tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + qq * WG_NC, v);
-            if (co < cout) {
-                float *dst = a.dW + ((size_t)co * cin + ci0 + WG_NC * j) * 9 + t;
+        for (int cq = warp >> 2; cq < WG_NC / 4; cq += 2) {
+            float v[9][4];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) atomicAdd(dst + 9 * i, v[i]);
+            for (int t = 0; t < 9; ++t)
+                tmem_ld4(tmem + ((uint32_t)(quarter * 32) << 16) + (t % 3) * WG_N + (t / 3) * WG_NC + 4 * cq, v[t]);
+            tmem_ld_wait();
+            if (!own) continue;
+            if (a.vec) {
+#pragma unroll
+                for (int k = 0; k < 9; ++k)   // value 4k + e is channel (4k + e) / 9, tap (4k + e) % 9
+                    red_add4(dst + 36 * cq + 4 * k, v[(4 * k) % 9][(4 * k) / 9], v[(4 * k + 1) % 9][(4 * k + 1) / 9],
+                             v[(4 * k + 2) % 9][(4 * k + 2) / 9], v[(4 * k + 3) % 9][(4 * k + 3) / 9]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 36; ++k) atomicAdd(dst + 36 * cq + k, v[k % 9][k / 9]);
             }
         }
     }
@@ -586,49 +575,38 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
     }
 }
 
-// One launch over `groups` channel groups of NCH chunks from input channel
-// a.ci_base on, in one wave of `per_sm` CTAs per SM (the buffers fill an SM's
-// shared memory): the CTAs of every (group, output block) split the tiles
-// evenly, at most per_sm * kSMs CTAs in all (a last wave of a few CTAs would
-// cost a whole run of tiles).
-template <int NCH, int R>
-int launch_wgrad_tc_t(WgArgs a, int groups, int coblocks, int per_sm, cudaStream_t st)
+// One launch in one wave of two CTAs per SM: the CTAs of every (chunk, output
+// block) split the tiles evenly (a last wave of a few CTAs would cost a whole
+// run of tiles), with at least WG_MIN_TILES each.
+template <int M, int R>
+int launch_wgrad_tc_t(WgArgs a, cudaStream_t st)
 {
-    const WgLayout L = wg_layout(NCH, R, std::min(a.cout, 128) >> 3);
-    const int xctas = std::max(1, per_sm * kSMs / (groups * coblocks));
-    a.tiles_per_cta = ceil_div(a.n_tiles, xctas);
-    auto kernel = wgrad_tc_kernel<NCH, R>;
+    const WgLayout L = wg_layout(M, R, std::min(a.cout, M) >> 3);
+    const int chunks = a.cin / WG_NC, coblocks = ceil_div(a.cout, M);
+    const int xctas = std::max(1, 2 * kSMs / (chunks * coblocks));
+    a.tiles_per_cta = std::max(ceil_div(a.n_tiles, xctas), WG_MIN_TILES);
+    auto kernel = wgrad_tc_kernel<M, R>;
     MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L.bytes));
     MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                       (int)cudaSharedmemCarveoutMaxShared));
-    const int ctas = ceil_div(a.n_tiles, a.tiles_per_cta);
-    kernel<<<dim3(ctas, groups, coblocks), WG_TC_THREADS, L.bytes, st>>>(a);
+    kernel<<<dim3(ceil_div(a.n_tiles, a.tiles_per_cta), chunks, coblocks), WG_TC_THREADS, L.bytes, st>>>(a);
     return MVS_OK;
 }
 
-// Shared memory one CTA may use at `per_sm` CTAs per SM.
-inline int wg_limit(int per_sm) { return per_sm == 1 ? WG_SMEM_MAX : WG_SMEM_SM / per_sm - 1024; }
-
-// The deepest raw ring that fits (at most 8 stages), or 0.
-inline int wg_stages(int nch, int cg, int per_sm)
+// The deepest ring of which two CTAs fit an SM.
+template <int M>
+int launch_wgrad_tc_m(const WgArgs &a, cudaStream_t st)
 {
-    for (int r = 8; r >= 2; --r)
-        if (wg_layout(nch, r, cg).bytes <= wg_limit(per_sm)) return r;
-    return 0;
-}
-
-template <int NCH>
-int launch_wgrad_tc_n(WgArgs a, int groups, int coblocks, int per_sm, cudaStream_t st)
-{
-    switch (wg_stages(NCH, std::min(a.cout, 128) >> 3, per_sm)) {
-    case 8: return launch_wgrad_tc_t<NCH, 8>(a, groups, coblocks, per_sm, st);
-    case 7: return launch_wgrad_tc_t<NCH, 7>(a, groups, coblocks, per_sm, st);
-    case 6: return launch_wgrad_tc_t<NCH, 6>(a, groups, coblocks, per_sm, st);
-    case 5: return launch_wgrad_tc_t<NCH, 5>(a, groups, coblocks, per_sm, st);
-    case 4: return launch_wgrad_tc_t<NCH, 4>(a, groups, coblocks, per_sm, st);
-    case 3: return launch_wgrad_tc_t<NCH, 3>(a, groups, coblocks, per_sm, st);
-    case 2: return launch_wgrad_tc_t<NCH, 2>(a, groups, coblocks, per_sm, st);
-    default: return set_error(MVS_ERR_ARG, "wgrad: %d chunks do not fit", NCH);
+    int r = WG_MAX_STAGES;
+    while (r > 2 && wg_layout(M, r, std::min(a.cout, M) >> 3).bytes > WG_SMEM_SM / 2 - 1024) --r;
+    switch (r) {
+    case 8: return launch_wgrad_tc_t<M, 8>(a, st);
+    case 7: return launch_wgrad_tc_t<M, 7>(a, st);
+    case 6: return launch_wgrad_tc_t<M, 6>(a, st);
+    case 5: return launch_wgrad_tc_t<M, 5>(a, st);
+    case 4: return launch_wgrad_tc_t<M, 4>(a, st);
+    case 3: return launch_wgrad_tc_t<M, 3>(a, st);
+    default: return launch_wgrad_tc_t<M, 2>(a, st);
     }
 }
 
@@ -636,26 +614,9 @@ int launch_wgrad_tc(const bf16 *x, int cin, const bf16 *dz, int cout, int B, int
                     cudaStream_t st)
 {
     if (cout % 8 || cin % WG_NC) return set_error(MVS_ERR_ARG, "wgrad: cin %d, cout %d", cin, cout);
-    WgArgs a{x, dz, dW, err, B, H, W, cin, cout, ceil_div(W, TW), ceil_div(H, TH), 1, 0, 0};
+    WgArgs a{x, dz, dW, err, B, H, W, cin, cout, ceil_div(W, TW), ceil_div(H, TH), 1, 0, ((uintptr_t)dW & 15) == 0};
     a.n_tiles = B * a.tiles_x * a.tiles_y;
-    const int chunks = cin / WG_NC, coblocks = ceil_div(cout, 128);
-    const int cg = std::min(cout, 128) >> 3;
-    // Two CTAs per SM, one chunk each, where one chunk's buffers and at least
-    // three raw stages fit in half an SM (16 output channels): the two CTAs'
-    // barrier-separated phases overlap.  Otherwise one CTA per SM: pairs of
-    // 16-channel chunks share a staged dz tile where two chunks' buffers and
-    // two raw stages fit, and an odd chunk runs alone.  (A single MMA buffer
-    // to fit two CTAs per SM at 32 and 64 output channels measured no faster.)
-    if (wg_stages(1, cg, 2) >= 3) return launch_wgrad_tc_n<1>(a, chunks, coblocks, 2, st);
-    const bool pairs = chunks >= 2 && wg_stages(2, cg, 1) >= 2;
-    if (pairs)
-        if (int rc = launch_wgrad_tc_n<2>(a, chunks / 2, coblocks, 1, st)) return rc;
-    const int first = pairs ? chunks & ~1 : 0;
-    if (first < chunks) {
-        a.ci_base = first * WG_NC;
-        if (int rc = launch_wgrad_tc_n<1>(a, chunks - first, coblocks, 1, st)) return rc;
-    }
-    return MVS_OK;
+    return cout <= 64 ? launch_wgrad_tc_m<64>(a, st) : launch_wgrad_tc_m<128>(a, st);
 }
 
 // ---------------------------------------------------------------------------
