@@ -13,9 +13,10 @@
 // channels, 16 bytes per pixel, which is exactly the "no swizzle, K-major"
 // operand layout (8 rows x 16 bytes per core matrix), so every tap's A operand
 // is the same halo addressed from a different start: no im2col copy.  The
-// weights of a slice are staged as [tap][8-ch plane][Cout][8].  Two stages
-// alternate: the copy of slice c+1 overlaps the MMAs of slice c, and an
-// mbarrier signalled by tcgen05.commit says when a stage may be refilled.
+// weights of a slice are staged as [tap][8-ch plane][Cout][8].  Up to three
+// stages form a ring: the copies of the next two slices overlap the MMAs of a
+// slice, and an mbarrier signalled by tcgen05.commit says when a stage may be
+// refilled.
 // The epilogue reads the accumulator with tcgen05.ld (one pixel per thread),
 // adds the bias, applies ReLU or the ReLU mask of the backward pass and
 // stores bf16.
@@ -117,9 +118,25 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool v
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0)
                  : "memory");
 }
+// untiled bulk copy (16-byte aligned, a multiple of 16 bytes), counted on `bar`
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) { return (uint32_t)f2bf(a) | ((uint32_t)f2bf(b) << 16); }
+// a in the low half, both rounded to nearest even (NaN stays NaN)
+__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b)
+{
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
+}
 
 // ---------------------------------------------------------------------------
 // 3x3 convolution, zero padding, on tensor cores
@@ -153,103 +170,130 @@ struct ConvSmem {
     static constexpr int HBYTES = 2 * HPIX * 16;          // two 8-channel planes
     static constexpr int W_BYTES = 9 * 2 * COUT * 16;
     static constexpr int STAGE = (HBYTES + W_BYTES + 127) / 128 * 128;
-    static constexpr int BYTES = 2 * STAGE + 64;
+    static constexpr int bytes(int stages) { return stages * STAGE + 64 + COUT * (int)sizeof(float); }
     static constexpr int TMEM_COLS = MT * COUT <= 32 ? 32 : MT * COUT <= 64 ? 64 : MT * COUT <= 128 ? 128 : 256;
 };
 
-template <int COUT, int MT = 1>
-__global__ void __launch_bounds__(CONV_THREADS) conv3x3_tc_kernel(ConvArgs a)
+// NST: stages of the ring, at most the number of 16-channel slices.
+template <int COUT, int MT, int NST>
+__global__ void __launch_bounds__(CONV_THREADS, NST == 1 ? 12 : NST == 2 ? 6 : 4) conv3x3_tc_kernel(ConvArgs a)
 {
     using S = ConvSmem<COUT, MT>;
     extern __shared__ __align__(128) unsigned char smem[];
     const int H = a.H, W = a.W, cin = a.cin;
     const int nslices = cin >> 4;
-    // one 16-channel slice needs one stage (launch_conv_t gives the CTA that much)
-    const int nstages = nslices > 1 ? 2 : 1;
-    uint64_t *bars = (uint64_t *)(smem + nstages * S::STAGE);
-    uint32_t *tmem_slot = (uint32_t *)(smem + nstages * S::STAGE + 16);
+    uint64_t *bars = (uint64_t *)(smem + NST * S::STAGE);   // the MMAs that read a stage are done
+    uint64_t *wbars = bars + NST;                           // a stage's weights have landed
+    uint32_t *tmem_slot = (uint32_t *)(bars + 2 * NST);
+    float *sbias = (float *)(smem + NST * S::STAGE + 64);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int b = blockIdx.y;
     const int tx = blockIdx.x % a.tiles_x, ty = blockIdx.x / a.tiles_x;
     const int x0 = tx * TW, y0 = ty * (MT * TH);
     const size_t img = (size_t)H * W;
-
-    if (warp == 0) tmem_alloc(tmem_slot, S::TMEM_COLS);
-    if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
     const uint32_t sbase = smem_u32(smem);
 
-    // stage slice c into buffer s: halo pixels (2 x 16 B) and 9 taps of weights
-    auto load = [&](int c, int s) {
+    // Each thread's halo copies are the same for every slice: 16-byte halves
+    // tid, tid + 128, ... of the halo pixels.
+    constexpr int HI = (2 * S::HPIX + CONV_THREADS - 1) / CONV_THREADS;
+    const bf16 *const origin = a.in + ((size_t)b * img + (size_t)y0 * W + x0) * cin + 8 * (tid & 1);
+    const bool inner = y0 > 0 && x0 > 0 && y0 + MT * TH < H && x0 + TW < W;   // the halo lies inside the image
+    // stage slice c in stage c % NST: halo pixels (2 x 16 B) by cp.async (one
+    // commit group), the 9 taps' weights by bulk copies (contiguous per tap)
+    // that signal the stage's wbar
+    auto load = [&](int c) {
+        const int s = c % NST;
         const uint32_t hb = sbase + s * S::STAGE, wb = hb + S::HBYTES;
-        for (int k = tid; k < 2 * S::HPIX; k += CONV_THREADS) {
+        const bf16 *src0 = origin + 16 * c;
+#pragma unroll
+        for (int i = 0; i < HI; ++i) {
+            const int k = tid + i * CONV_THREADS;
+            if (k >= 2 * S::HPIX) break;
             const int pix = k >> 1, half = k & 1;
-            const int hy = pix / HW_, hx = pix - hy * HW_;
-            const int gy = y0 - 1 + hy, gx = x0 - 1 + hx;
-            const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
-            const bf16 *src = a.in + ((size_t)b * img + (ok ? (size_t)gy * W + gx : 0)) * cin + 16 * c + 8 * half;
-            cp_async16(hb + (half * S::HPIX + pix) * 16, src, ok);
+            const int hy = pix / HW_ - 1, hx = pix - (hy + 1) * HW_ - 1;
+            const bool ok = inner || (y0 + hy >= 0 && y0 + hy < H && x0 + hx >= 0 && x0 + hx < W);
+            cp_async16(hb + (half * S::HPIX + pix) * 16, ok ? src0 + (hy * W + hx) * cin : a.in, ok);
         }
-        constexpr int WV = 2 * COUT;   // 16-byte vectors per tap
-        for (int k = tid; k < 9 * WV; k += CONV_THREADS) {
-            const int t = k / WV, r = k - t * WV;   // r = plane * COUT + co
-            const bf16 *src = a.wpack + ((size_t)(t * (cin >> 3) + 2 * c) * COUT) * 8 + (size_t)r * 8;
-            cp_async16(wb + (t * WV + r) * 16, src, true);
+        cp_async_commit();
+        if (warp == 1) {
+            constexpr uint32_t WB = 2 * COUT * 16;   // bytes per tap
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&wbars[s])),
+                             "r"(9 * WB)
+                             : "memory");
+            __syncwarp();
+            if (lane < 9)
+                bulk_copy(wb + lane * WB, a.wpack + ((size_t)(lane * (cin >> 3) + 2 * c) * COUT) * 8, WB, &wbars[s]);
         }
-        cp_async_wait_all();
-        fence_async_smem();
     };
+
+    if (warp == 0) tmem_alloc(tmem_slot, S::TMEM_COLS);
+    if (tid == 32) {
+        for (int k = 0; k < NST; ++k) mbar_init(&wbars[k], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) __syncwarp();
+    if (tid == 0) {
+        for (int k = 0; k < NST; ++k) mbar_init(&bars[k], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    constexpr int AHEAD = NST > 1 ? NST - 1 : 1;   // slices in flight before the first MMAs
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) load(k);
+    if (a.bias && tid < COUT) sbias[tid] = a.bias[tid];
+    if (COUT > CONV_THREADS && a.bias && tid + CONV_THREADS < COUT) sbias[tid + CONV_THREADS] = a.bias[tid + CONV_THREADS];
+    tc_fence_before();
 
     constexpr uint32_t idesc = idesc_bf16(128, COUT);
     bool failed = false;
-    load(0, 0);
-    __syncthreads();
+    int last = -1;   // the last slice whose MMAs were due (the same in every thread)
     for (int c = 0; c < nslices; ++c) {
-        const int s = c & 1;
-        if (tid == 0) {
+        cp_async_wait_group<AHEAD - 1>();   // slice c's halo landed
+        fence_async_smem();
+        failed = __syncthreads_or(failed) != 0;   // (the first one also publishes barriers, tensor memory and bias)
+        if (failed) break;
+        const int s = c % NST;
+        // (a weight copy that never lands leaves the MMAs out: the waits on
+        // bars[s] below then give up)
+        if (tid == 0 && mbar_wait_bounded(&wbars[s], (uint32_t)((c / NST) & 1), kWaitNs)) {
             tc_fence_after();
+            const uint32_t tmem = *tmem_slot;
+            // descriptors differ only in their start address (16-byte units)
             const uint32_t hb = sbase + s * S::STAGE, wb = hb + S::HBYTES;
+            const uint64_t ad = smem_desc(hb, S::HPIX * 16, HW_ * 16), bd = smem_desc(wb, COUT * 16, 128);
 #pragma unroll
             for (int t = 0; t < 9; ++t) {
                 const int ky = t / 3, kx = t - 3 * ky;
-                const uint64_t bd = smem_desc(wb + t * 2 * COUT * 16, COUT * 16, 128);
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    const uint64_t ad = smem_desc(hb + ((mt * TH + ky) * HW_ + kx) * 16, S::HPIX * 16, HW_ * 16);
-                    mma_bf16(tmem + (uint32_t)(mt * COUT), ad, bd, idesc, (c > 0 || t > 0) ? 1u : 0u);
-                }
+                for (int mt = 0; mt < MT; ++mt)
+                    mma_bf16(tmem + (uint32_t)(mt * COUT), ad + (mt * TH + ky) * HW_ + kx, bd + t * 2 * COUT, idesc,
+                             (c > 0 || t > 0) ? 1u : 0u);
             }
             mma_commit(&bars[s]);
         }
-        if (c + 1 < nslices) {
-            if (c >= 1) {
-                // stage s^1 was last read by the MMAs of slice c-1
-                const bool ok = mbar_wait_bounded(&bars[s ^ 1], ((c - 1) >> 1) & 1, kWaitNs);
-                failed = __syncthreads_or(!ok) != 0;
-                if (failed) break;
-            }
-            load(c + 1, s ^ 1);
-            __syncthreads();
+        last = c;
+        if (NST > 1 && c + AHEAD < nslices) {
+            // stage (c - 1) % NST takes slice c + NST - 1 once slice c - 1's MMAs have read it
+            failed = c >= 1 && !mbar_wait_bounded(&bars[(c - 1) % NST], (uint32_t)(((c - 1) / NST) & 1), kWaitNs);
+            if (!failed) load(c + AHEAD);
+        } else {
+            cp_async_commit();   // empty groups keep the group count per slice fixed
         }
     }
-    if (!failed) {
-        const int last = nslices - 1;
-        const bool ok = mbar_wait_bounded(&bars[last & 1], (last >> 1) & 1, kWaitNs);
-        failed = __syncthreads_or(!ok) != 0;
-    }
+    // one thread waits for the last MMAs, the others at the barrier (a wait of
+    // all of them took issue slots from the CTAs that share the SM)
+    if (tid == 0 && !failed) failed = !mbar_wait_bounded(&bars[last % NST], (uint32_t)((last / NST) & 1), kWaitNs);
+    failed = __syncthreads_or(failed) != 0;
+    const uint32_t tmem = *tmem_slot;
     if (failed) {
         if (tid == 0) atomicExch(a.err, 1);
-        // give the tensor core a second bounded chance to finish before the
-        // accumulator columns are released
-        const int last = nslices - 1;
-        mbar_wait_bounded(&bars[last & 1], (last >> 1) & 1, kWaitNs);
+        // give the tensor core and the copies a second bounded chance to finish
+        // before the accumulator columns are released
+        cp_async_wait_all();
+        if (last >= 0) mbar_wait_bounded(&bars[last % NST], (uint32_t)((last / NST) & 1), kWaitNs);
+        if (tid == 32)
+            for (int c = max(0, last); c < min(nslices, last + NST); ++c)
+                mbar_wait_bounded(&wbars[c % NST], (uint32_t)((c / NST) & 1), kWaitNs);
         tc_fence_before();
         __syncthreads();
         if (warp == 0) {
@@ -273,7 +317,7 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3x3_tc_kernel(ConvArgs a)
         tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * COUT + c0), v);
         if (a.bias) {
 #pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] += a.bias[c0 + k];
+            for (int k = 0; k < 16; ++k) v[k] += sbias[c0 + k];
         }
         if (a.relu) {
 #pragma unroll
@@ -306,17 +350,31 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3x3_tc_kernel(ConvArgs a)
     }
 }
 
+template <int COUT, int MT, int NST>
+int launch_conv_n(const ConvArgs &a, int B, cudaStream_t st)
+{
+    using S = ConvSmem<COUT, MT>;
+    auto kernel = conv3x3_tc_kernel<COUT, MT, NST>;
+    MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::bytes(NST)));
+    MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                      (int)cudaSharedmemCarveoutMaxShared));
+    const int tiles = a.tiles_x * ceil_div(a.H, MT * TH);
+    kernel<<<dim3(tiles, B), CONV_THREADS, S::bytes(NST), st>>>(a);
+    return MVS_OK;
+}
+
+// A ring of three stages, or as many as there are 16-channel slices: more CTAs
+// then share an SM.  Against two stages whose copies were waited for slice by
+// slice (batch 4, with the weight pack, B200): 192->64 at 160x120 47 -> 37 us,
+// 64->64 26 -> 22 us, 96->32 at 320x240 54 -> 47 us; one slice, 16->16 at
+// 640x480, 40 -> 37 us (fewer instructions per copied byte).
 template <int COUT, int MT = 1>
 int launch_conv_t(const ConvArgs &a, int B, cudaStream_t st)
 {
-    using S = ConvSmem<COUT, MT>;
-    MVS_TRY_CUDA(cudaFuncSetAttribute(conv3x3_tc_kernel<COUT, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      S::BYTES));
-    const int tiles = a.tiles_x * ceil_div(a.H, MT * TH);
-    // a 16-channel input is one slice: one stage, so more CTAs share an SM
-    const int bytes = a.cin > 16 ? S::BYTES : S::STAGE + 64;
-    conv3x3_tc_kernel<COUT, MT><<<dim3(tiles, B), CONV_THREADS, bytes, st>>>(a);
-    return MVS_OK;
+    static_assert(ConvSmem<COUT, MT>::bytes(3) <= 227 * 1024, "three stages fit a CTA");
+    if (a.cin <= 16) return launch_conv_n<COUT, MT, 1>(a, B, st);
+    if (a.cin <= 32) return launch_conv_n<COUT, MT, 2>(a, B, st);
+    return launch_conv_n<COUT, MT, 3>(a, B, st);
 }
 
 int launch_conv(const bf16 *in, int cin, const bf16 *wpack, const float *bias, const bf16 *mask, bf16 *out, int cout,
@@ -359,7 +417,7 @@ struct WgArgs {
     int vec;          // dW is 16-byte aligned
 };
 
-constexpr int WG_TC_THREADS = 256;
+constexpr int WG_COPY = 256, WG_TC_THREADS = WG_COPY + 32;   // eight copying warps and one that issues the MMAs
 constexpr int WG_NC = 16;                                      // input channels per chunk
 constexpr int WG_HALO_W = TW + 2, WG_HALO_H = TH + 2;          // 10 x 18 input pixels around an 8 x 16 tile
 constexpr int WG_HALO_BYTES = 2 * WG_HALO_H * WG_HALO_W * 16;  // 5760
@@ -388,10 +446,6 @@ __host__ __device__ inline WgLayout wg_layout(int m, int stages, int cg)
 
 // MN-major descriptors have the instruction descriptor's transpose bits set
 __host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N) { return idesc_bf16(M, N) | (1u << 15) | (1u << 16); }
-
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4])
 {
@@ -447,41 +501,60 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
     const uint32_t tmem = *tmem_slot;
     const uint32_t sbase = smem_u32(smem);
 
-    // Each thread's copies are the same for every tile: dz pixel (tid & 127) of
-    // the groups tid >> 7, + 2, ...; halo items tid, tid + 256 (halo pixel,
-    // then channel group), worked out once here.
+    // Each copying thread's copies are the same for every tile: dz pixel
+    // (tid & 127) of the groups tid >> 7, + 2, ...; halo items tid, tid + 256
+    // (halo pixel, then channel group), worked out once here.
     constexpr int HALO_ITEMS = 2 * WG_HALO_H * WG_HALO_W;
-    constexpr int HI = (HALO_ITEMS + WG_TC_THREADS - 1) / WG_TC_THREADS;
+    constexpr int HI = (HALO_ITEMS + WG_COPY - 1) / WG_COPY;
+    const bool copies = tid < WG_COPY;
     const int dz_m = tid & 127, dz_y = dz_m >> 3, dz_x = dz_m & 7, dz_g0 = tid >> 7;
     int h_y[HI], h_x[HI], h_dst[HI];
 #pragma unroll
     for (int i = 0; i < HI; ++i) {
-        const int k = tid + i * WG_TC_THREADS;
+        const int k = tid + i * WG_COPY;
         const int pix = k >> 1, g = k & 1, y = pix / WG_HALO_W, x = pix - y * WG_HALO_W;
         h_y[i] = y - 1;
         h_x[i] = x - 1;
         h_dst[i] = k < HALO_ITEMS ? ((y * 2 + g) * WG_HALO_W + x) * 16 : -1;
     }
-    const bf16 *xg = a.x + ci0 + 8 * (tid & 1);
-    // cp.async of tile `tile`'s dz and input halo into stage s (one commit group)
-    auto load = [&](int tile, int s) {
-        const int b = tile / (a.tiles_x * a.tiles_y), r = tile - b * a.tiles_x * a.tiles_y;
-        const int y0 = (r / a.tiles_x) * TH, x0 = (r % a.tiles_x) * TW;
-        const uint32_t ab = sbase + s * L.stage_bytes, hb = ab + L.a_bytes;
-        {
-            const int gy = y0 + dz_y, gx = x0 + dz_x;
-            const bool ok = gy < H && gx < W;
-            const bf16 *src = a.dz + ((size_t)b * img + (ok ? (size_t)gy * W + gx : 0)) * cout + co0 + 8 * dz_g0;
-            for (int g = dz_g0, i = 0; g < cg; g += 2, ++i) cp_async16(ab + (g * 128 + dz_m) * 16, src + 16 * i, ok);
-        }
+    int h_off[HI];
 #pragma unroll
-        for (int i = 0; i < HI; ++i) {
-            if (h_dst[i] < 0) continue;
-            const int gy = y0 + h_y[i], gx = x0 + h_x[i];
-            const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
-            cp_async16(hb + h_dst[i], xg + ((size_t)b * img + (ok ? (size_t)gy * W + gx : 0)) * cin, ok);
+    for (int i = 0; i < HI; ++i) h_off[i] = (h_y[i] * W + h_x[i]) * cin;
+    const int dz_off = (dz_y * W + dz_x) * cout;
+    const bf16 *xg = a.x + ci0 + 8 * (tid & 1);
+    const bf16 *zg = a.dz + co0 + 8 * dz_g0;
+    // the next tile to copy: image lb, tile row and column lty, ltx
+    const int per_img = a.tiles_x * a.tiles_y;
+    int lb = t_begin / per_img, lty = (t_begin - lb * per_img) / a.tiles_x,
+        ltx = t_begin - lb * per_img - lty * a.tiles_x;
+    // cp.async of the next tile's dz and input halo into stage s (one commit group)
+    auto load = [&](int s) {
+        const int y0 = lty * TH, x0 = ltx * TW;
+        const uint32_t ab = sbase + s * L.stage_bytes, hb = ab + L.a_bytes;
+        const size_t pb = (size_t)lb * img + (size_t)y0 * W + x0;
+        const bf16 *zt = zg + pb * cout + dz_off, *xt = xg + pb * cin;
+        uint32_t zd = ab + (dz_g0 * 128 + dz_m) * 16;
+        if (y0 > 0 && x0 > 0 && y0 + TH < H && x0 + TW < W) {   // halo and all inside the image
+            for (int g = dz_g0; g < cg; g += 2, zt += 16, zd += 2 * 128 * 16) cp_async16(zd, zt, true);
+#pragma unroll
+            for (int i = 0; i < HI; ++i)
+                if (h_dst[i] >= 0) cp_async16(hb + h_dst[i], xt + h_off[i], true);
+        } else {
+            const bool ok = y0 + dz_y < H && x0 + dz_x < W;
+            if (!ok) zt = a.dz;
+            for (int g = dz_g0; g < cg; g += 2, zt += ok ? 16 : 0, zd += 2 * 128 * 16) cp_async16(zd, zt, ok);
+#pragma unroll
+            for (int i = 0; i < HI; ++i) {
+                const int gy = y0 + h_y[i], gx = x0 + h_x[i];
+                const bool in = gy >= 0 && gy < H && gx >= 0 && gx < W;
+                if (h_dst[i] >= 0) cp_async16(hb + h_dst[i], in ? xt + h_off[i] : a.x, in);
+            }
         }
         cp_async_commit();
+        if (++ltx == a.tiles_x) {
+            ltx = 0;
+            if (++lty == a.tiles_y) lty = 0, ++lb;
+        }
     };
 
     constexpr uint32_t idesc = idesc_bf16_mn(M, WG_N);
@@ -489,7 +562,7 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
     bool failed = false;
     int last = -1;   // the last tile whose MMAs were issued (the same in every thread)
     for (int k = 0; k < R - 1; ++k) {
-        if (k < n) load(t_begin + k, k);
+        if (k < n && copies) load(k);
         else cp_async_commit();   // empty groups keep the group count per tile fixed
     }
     // tile c's MMAs read stage c % R and signal bars[c % R]: that barrier's
@@ -499,25 +572,24 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
         fence_async_smem();             // visible to the MMAs
         failed = __syncthreads_or(failed) != 0;
         if (failed) break;
-        if (tid == 0) {
+        if (tid == WG_COPY) {
             tc_fence_after();
+            // descriptors differ only in their start address (16-byte units)
             const uint32_t ab = sbase + (c % R) * L.stage_bytes, hb = ab + L.a_bytes;
+            const uint64_t ad = smem_desc(ab, 128, 128 * 16), bd = smem_desc(hb, 2 * WG_HALO_W * 16, WG_HALO_W * 16);
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {
-                const uint64_t ad = smem_desc(ab + ks * 256, 128, 128 * 16);
+            for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
-                for (int kx = 0; kx < 3; ++kx) {
-                    const uint64_t bd = smem_desc(hb + (4 * ks * WG_HALO_W + kx) * 16, 2 * WG_HALO_W * 16, WG_HALO_W * 16);
-                    mma_bf16(tmem + kx * WG_N, ad, bd, idesc, (c > 0 || ks > 0) ? 1u : 0u);
-                }
-            }
+                for (int kx = 0; kx < 3; ++kx)
+                    mma_bf16(tmem + kx * WG_N, ad + 16 * ks, bd + 4 * ks * WG_HALO_W + kx, idesc,
+                             (c > 0 || ks > 0) ? 1u : 0u);
             mma_commit(&bars[c % R]);
         }
         last = c;
-        if (c + R - 1 < n) {
+        if (c + R - 1 < n && copies) {
             // stage (c - 1) % R takes tile c + R - 1 once tile c - 1's MMAs have read it
             failed = c >= 1 && !mbar_wait_bounded(&bars[(c - 1) % R], (uint32_t)(((c - 1) / R) & 1), kWaitNs);
-            if (!failed) load(t_begin + c + R - 1, (c + R - 1) % R);
+            if (!failed) load((c + R - 1) % R);
         } else {
             cp_async_commit();
         }
@@ -549,7 +621,7 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
         const bool own = (M == 128 || lane < 16) && co0 + row < cout;
         float *dst = a.dW + ((size_t)(co0 + row) * cin + ci0) * 9;
 #pragma unroll 1
-        for (int cq = warp >> 2; cq < WG_NC / 4; cq += 2) {
+        for (int cq = warp >> 2; cq < WG_NC / 4 && copies; cq += 2) {
             float v[9][4];
 #pragma unroll
             for (int t = 0; t < 9; ++t)
