@@ -142,14 +142,62 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b)
 // 3x3 convolution, zero padding, on tensor cores
 // ---------------------------------------------------------------------------
 
+// An activation tensor of `channels` channels at H x W: one tensor [B][H][W][channels],
+// or (up > 0) the concatenation that a decoder level reads, never stored: the
+// first `up` channels are the next coarser level's [B][H/2][W/2][up], nearest
+// upsampled, the others `skip` [B][H][W][channels - up].  H and W are even there.
+struct Act {
+    const bf16 *p, *skip;
+    int channels, up;
+};
+
+// Where 16 channels of an Act lie, from channel `c` on (a multiple of 16; `up`
+// is one too): base pointer, channels per pixel, and 1 for the coarser level.
+struct Source {
+    const bf16 *p;
+    int pitch, half;
+};
+__device__ __forceinline__ Source act_source(const Act &a, int c)
+{
+    if (a.up == 0) return Source{a.p + c, a.channels, 0};
+    if (c < a.up) return Source{a.p + c, a.up, 1};
+    return Source{a.skip + (c - a.up), a.channels - a.up, 0};
+}
+// Offset (in elements) of pixel (y + dy, x + dx) from pixel (y, x) of image b, y and
+// x even, and of that pixel itself.
+__device__ __forceinline__ int source_delta(const Source &s, int W, int dy, int dx)
+{
+    return ((dy >> s.half) * (W >> s.half) + (dx >> s.half)) * s.pitch;
+}
+__device__ __forceinline__ size_t source_at(const Source &s, int H, int W, int b, int y, int x)
+{
+    return (((size_t)b * (H >> s.half) + (y >> s.half)) * (W >> s.half) + (x >> s.half)) * s.pitch;
+}
+
+struct Norm {
+    float depth_scale, depth_shift;   // channel 0 = depth * scale + shift
+    float cost_clip;                  // channel 1 = 1 - min(cost, clip)
+    float u_scale, v_scale;           // u = wta + u_scale * out0, v = v_scale * out{1,2}
+    float w_u, w_v;                   // loss weights of (u - u*)^2 and |v - v*|^2
+};
+
+// The 1x1 head on the last activation (16 channels), formed in that
+// convolution's epilogue; u null: no head.
+struct Head {
+    const float *w, *b, *wta;   // [3][16], [3], [B][H][W]
+    float *u, *v;               // [B][H][W], [B][2][H][W]
+    Norm nm;
+};
+
 struct ConvArgs {
-    const bf16 *in;     // [B][H][W][cin]
+    Act in;             // cin channels
     const bf16 *wpack;  // [9][cin/8][COUT][8]
     const float *bias;  // [COUT] or null
-    const bf16 *mask;   // [B][H][W][COUT] or null: out *= (mask > 0)
+    Act mask;           // COUT channels, or p null; out *= (mask > 0)
     bf16 *out;          // [B][H][W][COUT]
     int *err;           // set to 1 when a bounded wait gives up
     int H, W, cin, relu, tiles_x;
+    Head head;
 };
 
 constexpr uint64_t kWaitNs = 1000000000ull;   // 1 s
@@ -196,7 +244,6 @@ __global__ void __launch_bounds__(CONV_THREADS, NST == 1 ? 12 : NST == 2 ? 6 : 4
     // Each thread's halo copies are the same for every slice: 16-byte halves
     // tid, tid + 128, ... of the halo pixels.
     constexpr int HI = (2 * S::HPIX + CONV_THREADS - 1) / CONV_THREADS;
-    const bf16 *const origin = a.in + ((size_t)b * img + (size_t)y0 * W + x0) * cin + 8 * (tid & 1);
     const bool inner = y0 > 0 && x0 > 0 && y0 + MT * TH < H && x0 + TW < W;   // the halo lies inside the image
     // stage slice c in stage c % NST: halo pixels (2 x 16 B) by cp.async (one
     // commit group), the 9 taps' weights by bulk copies (contiguous per tap)
@@ -204,7 +251,8 @@ __global__ void __launch_bounds__(CONV_THREADS, NST == 1 ? 12 : NST == 2 ? 6 : 4
     auto load = [&](int c) {
         const int s = c % NST;
         const uint32_t hb = sbase + s * S::STAGE, wb = hb + S::HBYTES;
-        const bf16 *src0 = origin + 16 * c;
+        const Source sr = act_source(a.in, 16 * c);
+        const bf16 *src0 = sr.p + source_at(sr, H, W, b, y0, x0) + 8 * (tid & 1);
 #pragma unroll
         for (int i = 0; i < HI; ++i) {
             const int k = tid + i * CONV_THREADS;
@@ -212,7 +260,7 @@ __global__ void __launch_bounds__(CONV_THREADS, NST == 1 ? 12 : NST == 2 ? 6 : 4
             const int pix = k >> 1, half = k & 1;
             const int hy = pix / HW_ - 1, hx = pix - (hy + 1) * HW_ - 1;
             const bool ok = inner || (y0 + hy >= 0 && y0 + hy < H && x0 + hx >= 0 && x0 + hx < W);
-            cp_async16(hb + (half * S::HPIX + pix) * 16, ok ? src0 + (hy * W + hx) * cin : a.in, ok);
+            cp_async16(hb + (half * S::HPIX + pix) * 16, ok ? src0 + source_delta(sr, W, hy, hx) : a.in.p, ok);
         }
         cp_async_commit();
         if (warp == 1) {
@@ -238,6 +286,12 @@ __global__ void __launch_bounds__(CONV_THREADS, NST == 1 ? 12 : NST == 2 ? 6 : 4
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     constexpr int AHEAD = NST > 1 ? NST - 1 : 1;   // slices in flight before the first MMAs
+    // dependent launch: the previous kernels are complete.  (The next grid is let
+    // in only here, once this CTA holds its tensor memory: CTAs that wait must not
+    // take it from CTAs that run.)
+    __syncthreads();
+    wait_for_previous_grid();
+    allow_next_grid();
 #pragma unroll
     for (int k = 0; k < AHEAD; ++k) load(k);
     if (a.bias && tid < COUT) sbias[tid] = a.bias[tid];
@@ -323,8 +377,9 @@ __global__ void __launch_bounds__(CONV_THREADS, NST == 1 ? 12 : NST == 2 ? 6 : 4
 #pragma unroll
             for (int k = 0; k < 16; ++k) v[k] = fmaxf(v[k], 0.f);
         }
-        if (a.mask && inside) {
-            const uint4 *mp = (const uint4 *)(a.mask + pidx * COUT + c0);
+        if (a.mask.p && inside) {
+            const Source sm = act_source(a.mask, c0);
+            const uint4 *mp = (const uint4 *)(sm.p + source_at(sm, H, W, b, py, px));
             const uint4 m0 = mp[0], m1 = mp[1];
             const uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
 #pragma unroll
@@ -335,10 +390,34 @@ __global__ void __launch_bounds__(CONV_THREADS, NST == 1 ? 12 : NST == 2 ? 6 : 4
         }
         if (inside) {
             uint4 *op = (uint4 *)(a.out + pidx * COUT + c0);
-            op[0] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
-                               pack_bf16x2(v[6], v[7]));
-            op[1] = make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]), pack_bf16x2(v[12], v[13]),
-                               pack_bf16x2(v[14], v[15]));
+            const uint4 o0 = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                                        pack_bf16x2(v[6], v[7]));
+            const uint4 o1 = make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]), pack_bf16x2(v[12], v[13]),
+                                        pack_bf16x2(v[14], v[15]));
+            op[0] = o0;
+            op[1] = o1;
+            if (COUT == 16 && a.head.u) {
+                // the head reads the stored (rounded) activation
+                const uint32_t ow[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
+                float o[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) o[k] = __ldg(a.head.b + k);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float lo = bf2f((uint16_t)(ow[j] & 0xffffu)), hi = bf2f((uint16_t)(ow[j] >> 16));
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        o[k] = fmaf(__ldg(a.head.w + 16 * k + 2 * j), lo, o[k]);
+                        o[k] = fmaf(__ldg(a.head.w + 16 * k + 2 * j + 1), hi, o[k]);
+                    }
+                }
+                float dw = __ldg(a.head.wta + pidx);
+                if (!(dw == dw)) dw = 0.f;
+                a.head.u[pidx] = dw + a.head.nm.u_scale * o[0];
+                float *vv = a.head.v + pidx + (size_t)b * img;   // [b][2][H][W]
+                vv[0] = a.head.nm.v_scale * o[1];
+                vv[img] = a.head.nm.v_scale * o[2];
+            }
         }
     }
     }
@@ -359,7 +438,7 @@ int launch_conv_n(const ConvArgs &a, int B, cudaStream_t st)
     MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                       (int)cudaSharedmemCarveoutMaxShared));
     const int tiles = a.tiles_x * ceil_div(a.H, MT * TH);
-    kernel<<<dim3(tiles, B), CONV_THREADS, S::bytes(NST), st>>>(a);
+    MVS_TRY_CUDA(launch_dependent(kernel, dim3(tiles, B), dim3(CONV_THREADS), S::bytes(NST), st, a));
     return MVS_OK;
 }
 
@@ -377,11 +456,12 @@ int launch_conv_t(const ConvArgs &a, int B, cudaStream_t st)
     return launch_conv_n<COUT, MT, 3>(a, B, st);
 }
 
-int launch_conv(const bf16 *in, int cin, const bf16 *wpack, const float *bias, const bf16 *mask, bf16 *out, int cout,
-                int B, int H, int W, int relu, int *err, cudaStream_t st)
+int launch_conv(const Act &in, const bf16 *wpack, const float *bias, const Act &mask, bf16 *out, int cout, int B, int H,
+                int W, int relu, int *err, cudaStream_t st, const Head &head = Head{})
 {
+    const int cin = in.channels;
     if (cin <= 0 || cin % 16 || cin > 512) return set_error(MVS_ERR_ARG, "conv input channels %d (multiple of 16)", cin);
-    ConvArgs a{in, wpack, bias, mask, out, err, H, W, cin, relu, ceil_div(W, TW)};
+    ConvArgs a{in, wpack, bias, mask, out, err, H, W, cin, relu, ceil_div(W, TW), head};
     switch (cout) {
     case 16: return launch_conv_t<16, CONV_MT16>(a, B, st);
     case 32: return launch_conv_t<32, CONV_MT32>(a, B, st);
@@ -409,7 +489,7 @@ int launch_conv(const bf16 *in, int cin, const bf16 *wpack, const float *bias, c
 // ---------------------------------------------------------------------------
 
 struct WgArgs {
-    const bf16 *x;    // [B][H][W][cin]
+    Act x;            // cin channels
     const bf16 *dz;   // [B][H][W][cout]
     float *dW;        // [cout][cin][9]
     int *err;
@@ -498,6 +578,10 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // dependent launch: the previous kernels are complete.  (The next grid is let
+    // in only here, once this CTA holds its tensor memory, as in the convolution.)
+    wait_for_previous_grid();
+    allow_next_grid();
     const uint32_t tmem = *tmem_slot;
     const uint32_t sbase = smem_u32(smem);
 
@@ -517,11 +601,12 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
         h_x[i] = x - 1;
         h_dst[i] = k < HALO_ITEMS ? ((y * 2 + g) * WG_HALO_W + x) * 16 : -1;
     }
+    const Source sx = act_source(a.x, ci0);
     int h_off[HI];
 #pragma unroll
-    for (int i = 0; i < HI; ++i) h_off[i] = (h_y[i] * W + h_x[i]) * cin;
+    for (int i = 0; i < HI; ++i) h_off[i] = source_delta(sx, W, h_y[i], h_x[i]);
     const int dz_off = (dz_y * W + dz_x) * cout;
-    const bf16 *xg = a.x + ci0 + 8 * (tid & 1);
+    const bf16 *xg = sx.p + 8 * (tid & 1);
     const bf16 *zg = a.dz + co0 + 8 * dz_g0;
     // the next tile to copy: image lb, tile row and column lty, ltx
     const int per_img = a.tiles_x * a.tiles_y;
@@ -532,7 +617,7 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
         const int y0 = lty * TH, x0 = ltx * TW;
         const uint32_t ab = sbase + s * L.stage_bytes, hb = ab + L.a_bytes;
         const size_t pb = (size_t)lb * img + (size_t)y0 * W + x0;
-        const bf16 *zt = zg + pb * cout + dz_off, *xt = xg + pb * cin;
+        const bf16 *zt = zg + pb * cout + dz_off, *xt = xg + source_at(sx, H, W, lb, y0, x0);
         uint32_t zd = ab + (dz_g0 * 128 + dz_m) * 16;
         if (y0 > 0 && x0 > 0 && y0 + TH < H && x0 + TW < W) {   // halo and all inside the image
             for (int g = dz_g0; g < cg; g += 2, zt += 16, zd += 2 * 128 * 16) cp_async16(zd, zt, true);
@@ -547,7 +632,7 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
             for (int i = 0; i < HI; ++i) {
                 const int gy = y0 + h_y[i], gx = x0 + h_x[i];
                 const bool in = gy >= 0 && gy < H && gx >= 0 && gx < W;
-                if (h_dst[i] >= 0) cp_async16(hb + h_dst[i], in ? xt + h_off[i] : a.x, in);
+                if (h_dst[i] >= 0) cp_async16(hb + h_dst[i], in ? xt + h_off[i] : a.x.p, in);
             }
         }
         cp_async_commit();
@@ -661,7 +746,8 @@ int launch_wgrad_tc_t(WgArgs a, cudaStream_t st)
     MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L.bytes));
     MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                       (int)cudaSharedmemCarveoutMaxShared));
-    kernel<<<dim3(ceil_div(a.n_tiles, a.tiles_per_cta), chunks, coblocks), WG_TC_THREADS, L.bytes, st>>>(a);
+    MVS_TRY_CUDA(launch_dependent(kernel, dim3(ceil_div(a.n_tiles, a.tiles_per_cta), chunks, coblocks),
+                                  dim3(WG_TC_THREADS), L.bytes, st, a));
     return MVS_OK;
 }
 
@@ -682,9 +768,9 @@ int launch_wgrad_tc_m(const WgArgs &a, cudaStream_t st)
     }
 }
 
-int launch_wgrad_tc(const bf16 *x, int cin, const bf16 *dz, int cout, int B, int H, int W, float *dW, int *err,
-                    cudaStream_t st)
+int launch_wgrad_tc(const Act &x, const bf16 *dz, int cout, int B, int H, int W, float *dW, int *err, cudaStream_t st)
 {
+    const int cin = x.channels;
     if (cout % 8 || cin % WG_NC) return set_error(MVS_ERR_ARG, "wgrad: cin %d, cout %d", cin, cout);
     WgArgs a{x, dz, dW, err, B, H, W, cin, cout, ceil_div(W, TW), ceil_div(H, TH), 1, 0, ((uintptr_t)dW & 15) == 0};
     a.n_tiles = B * a.tiles_x * a.tiles_y;
@@ -761,6 +847,8 @@ __global__ void __launch_bounds__(WG_THREADS) wgrad_kernel(const bf16 *__restric
 __global__ void __launch_bounds__(256) bgrad_kernel(const bf16 *__restrict__ dz, long long npix, int cout,
                                                     int px_per_cta, float *__restrict__ db)
 {
+    wait_for_previous_grid();   // dependent launch
+    allow_next_grid();
     __shared__ float red[256][9];   // 9: no bank conflicts
     const int tid = threadIdx.x, groups = cout >> 3;
     const long long p0 = (long long)blockIdx.x * px_per_cta, p1 = min(p0 + px_per_cta, npix);
@@ -796,18 +884,20 @@ __global__ void __launch_bounds__(256) bgrad_kernel(const bf16 *__restrict__ dz,
 int launch_wgrad_cuda_cores(const bf16 *x, int cin, const bf16 *dz, int cout, int B, int H, int W, float *dW,
                             cudaStream_t st);
 
-int launch_wgrad(const bf16 *x, int cin, const bf16 *dz, int cout, int B, int H, int W, float *dW, float *db, int *err,
+// (the CUDA-core form takes one tensor only)
+int launch_wgrad(const Act &x, const bf16 *dz, int cout, int B, int H, int W, float *dW, float *db, int *err,
                  cudaStream_t st, bool tensor_cores = true)
 {
     const long long npix = (long long)B * H * W;
     if (tensor_cores) {
-        MVS_RC_(launch_wgrad_tc(x, cin, dz, cout, B, H, W, dW, err, st));
+        MVS_RC_(launch_wgrad_tc(x, dz, cout, B, H, W, dW, err, st));
     } else {
-        MVS_RC_(launch_wgrad_cuda_cores(x, cin, dz, cout, B, H, W, dW, st));
+        MVS_RC_(launch_wgrad_cuda_cores(x.p, x.channels, dz, cout, B, H, W, dW, st));
     }
     if (db) {
         const int px = (int)std::max<long long>(256, (npix + 4 * kSMs - 1) / (4 * kSMs));
-        bgrad_kernel<<<(int)((npix + px - 1) / px), 256, 0, st>>>(dz, npix, cout, px, db);
+        MVS_TRY_CUDA(launch_dependent(bgrad_kernel, dim3((unsigned)((npix + px - 1) / px)), dim3(256), 0, st, dz, npix,
+                                      cout, px, db));
     }
     return MVS_OK;
 }
@@ -852,6 +942,8 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8])
 // 2x2 average pool: out [B][H/2][W/2][C]
 __global__ void pool_kernel(const bf16 *__restrict__ in, int B, int H, int W, int C, bf16 *__restrict__ out)
 {
+    wait_for_previous_grid();   // dependent launch
+    allow_next_grid();
     const int C8 = C >> 3, Ho = H >> 1, Wo = W >> 1;
     const long long n = (long long)B * Ho * Wo * C8;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
@@ -878,6 +970,8 @@ __global__ void pool_kernel(const bf16 *__restrict__ in, int B, int H, int W, in
 __global__ void pool_back_kernel(const bf16 *__restrict__ dp, const bf16 *__restrict__ dc, int ctot, int coff,
                                  const bf16 *__restrict__ e, int B, int H, int W, int C, bf16 *__restrict__ de)
 {
+    wait_for_previous_grid();   // dependent launch
+    allow_next_grid();
     const int C8 = C >> 3;
     const long long n = (long long)B * H * W * C8;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
@@ -901,31 +995,13 @@ __global__ void pool_back_kernel(const bf16 *__restrict__ dp, const bf16 *__rest
     }
 }
 
-// concat(nearest-upsampled prev (cp channels, H/2 x W/2), skip (cs channels))
-__global__ void upcat_kernel(const bf16 *__restrict__ prev, int cp, const bf16 *__restrict__ skip, int cs, int B,
-                             int H, int W, bf16 *__restrict__ out)
-{
-    const int ct8 = (cp + cs) >> 3;
-    const long long n = (long long)B * H * W * ct8;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const int c8 = (int)(k % ct8);
-        const long long p = k / ct8;
-        const int x = (int)(p % W), y = (int)((p / W) % H), b = (int)(p / ((long long)W * H));
-        const int c = 8 * c8;
-        uint4 v;
-        if (c < cp)
-            v = *(const uint4 *)(prev + (((size_t)b * (H >> 1) + (y >> 1)) * (W >> 1) + (x >> 1)) * cp + c);
-        else
-            v = *(const uint4 *)(skip + (size_t)p * cs + (c - cp));
-        *(uint4 *)(out + (size_t)k * 8) = v;
-    }
-}
-
 // gradient of the upsampled half: dprev[y][x] = sum of the 2x2 block of dc
 // (already masked by the concat's ReLU mask, which is prev's)
 __global__ void upcat_back_kernel(const bf16 *__restrict__ dc, int ctot, int B, int H, int W, int cp,
                                   bf16 *__restrict__ dprev)
 {
+    wait_for_previous_grid();   // dependent launch
+    allow_next_grid();
     const int C8 = cp >> 3, Hp = H >> 1, Wp = W >> 1;
     const long long n = (long long)B * Hp * Wp * C8;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
@@ -948,16 +1024,11 @@ __global__ void upcat_back_kernel(const bf16 *__restrict__ dc, int ctot, int B, 
 // input features, prediction head and loss
 // ---------------------------------------------------------------------------
 
-struct Norm {
-    float depth_scale, depth_shift;   // channel 0 = depth * scale + shift
-    float cost_clip;                  // channel 1 = 1 - min(cost, clip)
-    float u_scale, v_scale;           // u = wta + u_scale * out0, v = v_scale * out{1,2}
-    float w_u, w_v;                   // loss weights of (u - u*)^2 and |v - v*|^2
-};
-
 __global__ void features_kernel(const float *__restrict__ wta, const float *__restrict__ cost,
                                 const float *__restrict__ ref255, long long npix, Norm nm, bf16 *__restrict__ x0)
 {
+    wait_for_previous_grid();   // dependent launch
+    allow_next_grid();
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npix; p += (long long)gridDim.x * blockDim.x) {
         float d = wta[p];
         if (!(d == d)) d = 0.f;
@@ -969,40 +1040,6 @@ __global__ void features_kernel(const float *__restrict__ wta, const float *__re
         uint4 *o = (uint4 *)(x0 + (size_t)p * 16);
         o[0] = pack8(f);
         o[1] = pack8(z);
-    }
-}
-
-// u, v from the last decoder activation d (16 channels) by the 1x1 head
-__global__ void head_kernel(const bf16 *__restrict__ d, const float *__restrict__ Wh, const float *__restrict__ bh,
-                            const float *__restrict__ wta, long long npix, long long img, Norm nm,
-                            float *__restrict__ u, float *__restrict__ v)
-{
-    __shared__ float w[51];
-    if (threadIdx.x < 48) w[threadIdx.x] = Wh[threadIdx.x];
-    if (threadIdx.x < 3) w[48 + threadIdx.x] = bh[threadIdx.x];
-    __syncthreads();
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npix; p += (long long)gridDim.x * blockDim.x) {
-        float a[16], t[8];
-        unpack8(*(const uint4 *)(d + (size_t)p * 16), t);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = t[j];
-        unpack8(*(const uint4 *)(d + (size_t)p * 16 + 8), t);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) a[8 + j] = t[j];
-        float o[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            float s = w[48 + k];
-#pragma unroll
-            for (int c = 0; c < 16; ++c) s = fmaf(w[16 * k + c], a[c], s);
-            o[k] = s;
-        }
-        const long long b = p / img, q = p - b * img;
-        float dw = wta[p];
-        if (!(dw == dw)) dw = 0.f;
-        u[p] = dw + nm.u_scale * o[0];
-        v[(size_t)b * 2 * img + q] = nm.v_scale * o[1];
-        v[(size_t)b * 2 * img + img + q] = nm.v_scale * o[2];
     }
 }
 
@@ -1100,17 +1137,38 @@ __global__ void adam_kernel(float *__restrict__ w, const float *__restrict__ g, 
 }
 
 // W [cout][cin][9] (FP32) -> forward pack [9][cin/8][cout][8] and the
-// backward-data pack [9][cout/8][cin][8] of the flipped, transposed kernel
-__global__ void pack_kernel(const float *__restrict__ Wt, int cin, int cout, bf16 *__restrict__ fwd,
-                            bf16 *__restrict__ bwd)
+// backward-data pack [9][cout/8][cin][8] of the flipped, transposed kernel;
+// one grid row per layer.
+struct PackLayer {
+    const float *w;
+    bf16 *fwd, *bwd;   // bwd may be null
+    int cin, cout;
+};
+constexpr int PACK_LAYERS = 14;
+struct PackArgs {
+    PackLayer l[PACK_LAYERS];
+};
+__global__ void pack_kernel(PackArgs a)
 {
-    const int n = 9 * cin * cout;
+    wait_for_previous_grid();   // dependent launch
+    allow_next_grid();
+    const PackLayer &L = a.l[blockIdx.y];
+    const int cin = L.cin, cout = L.cout, n = 9 * cin * cout;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const int t = k % 9, ci = (k / 9) % cin, co = k / (9 * cin);
-        const uint16_t b = f2bf(Wt[k]);
-        fwd[(((size_t)t * (cin >> 3) + (ci >> 3)) * cout + co) * 8 + (ci & 7)] = b;
-        if (bwd) bwd[(((size_t)(8 - t) * (cout >> 3) + (co >> 3)) * cin + ci) * 8 + (co & 7)] = b;
+        const uint16_t b = f2bf(L.w[k]);
+        L.fwd[(((size_t)t * (cin >> 3) + (ci >> 3)) * cout + co) * 8 + (ci & 7)] = b;
+        if (L.bwd) L.bwd[(((size_t)(8 - t) * (cout >> 3) + (co >> 3)) * cin + ci) * 8 + (co & 7)] = b;
     }
+}
+
+// the packs of one layer
+int launch_pack(const float *w, int cin, int cout, bf16 *fwd, bf16 *bwd, cudaStream_t st)
+{
+    PackArgs p{};
+    p.l[0] = PackLayer{w, fwd, bwd, cin, cout};
+    MVS_TRY_CUDA(launch_dependent(pack_kernel, dim3(ceil_div(9 * cin * cout, 256)), dim3(256), 0, st, p));
+    return MVS_OK;
 }
 
 }  // namespace unet
@@ -1146,7 +1204,7 @@ struct mvs_unet {
     float *params = nullptr, *grads = nullptr, *adam_m = nullptr, *adam_v = nullptr;
     bf16 *packs = nullptr;
     // activations (and their gradients, prefixed g)
-    bf16 *x0, *e0a, *e0, *p0, *e1a, *e1, *p1, *e2a, *e2, *p2, *e3a, *e3, *c2, *d2a, *d2, *c1, *d1a, *d1, *c0, *d0a, *d0;
+    bf16 *x0, *e0a, *e0, *p0, *e1a, *e1, *p1, *e2a, *e2, *p2, *e3a, *e3, *d2a, *d2, *d1a, *d1, *d0a, *d0;
     bf16 *gd0, *gd0a, *gc0, *gd1, *gd1a, *gc1, *gd2, *gd2a, *gc2, *ge3, *ge3a, *gp2, *ge2, *ge2a, *gp1, *ge1, *ge1a,
         *gp0, *ge0, *ge0a;
     float *u = nullptr, *v = nullptr;   // predictions
@@ -1202,8 +1260,7 @@ int alloc_net(mvs_unet *n)
         {&n->x0, px(0) * 16},   {&n->e0a, px(0) * 16},  {&n->e0, px(0) * 16},   {&n->p0, px(1) * 16},
         {&n->e1a, px(1) * 32},  {&n->e1, px(1) * 32},   {&n->p1, px(2) * 32},   {&n->e2a, px(2) * 64},
         {&n->e2, px(2) * 64},   {&n->p2, px(3) * 64},   {&n->e3a, px(3) * 128}, {&n->e3, px(3) * 128},
-        {&n->c2, px(2) * 192},  {&n->d2a, px(2) * 64},  {&n->d2, px(2) * 64},   {&n->c1, px(1) * 96},
-        {&n->d1a, px(1) * 32},  {&n->d1, px(1) * 32},   {&n->c0, px(0) * 48},   {&n->d0a, px(0) * 16},
+        {&n->d2a, px(2) * 64},  {&n->d2, px(2) * 64},   {&n->d1a, px(1) * 32},  {&n->d1, px(1) * 32},    {&n->d0a, px(0) * 16},
         {&n->d0, px(0) * 16},   {&n->gd0, px(0) * 16},  {&n->gd0a, px(0) * 16}, {&n->gc0, px(0) * 48},
         {&n->gd1, px(1) * 32},  {&n->gd1a, px(1) * 32}, {&n->gc1, px(1) * 96},  {&n->gd2, px(2) * 64},
         {&n->gd2a, px(2) * 64}, {&n->gc2, px(2) * 192}, {&n->ge3, px(3) * 128}, {&n->ge3a, px(3) * 128},
@@ -1230,11 +1287,15 @@ int alloc_net(mvs_unet *n)
 
 int repack(mvs_unet *n, cudaStream_t st)
 {
+    static_assert(NCONV == PACK_LAYERS, "one pack entry per layer");
+    PackArgs p{};
+    int most = 0;
     for (int l = 0; l < NCONV; ++l) {
         const ConvLayer &c = n->L[l];
-        const int cnt = 9 * c.cin * c.cout;
-        pack_kernel<<<ceil_div(cnt, 256), 256, 0, st>>>(n->params + c.w_off, c.cin, c.cout, c.wf, l == E0A ? nullptr : c.wb);
+        most = std::max(most, 9 * c.cin * c.cout);
+        p.l[l] = PackLayer{n->params + c.w_off, c.wf, l == E0A ? nullptr : c.wb, c.cin, c.cout};
     }
+    MVS_TRY_CUDA(launch_dependent(pack_kernel, dim3(std::min(ceil_div(most, 256), kSMs), NCONV), dim3(256), 0, st, p));
     return check_launch("unet weight pack");
 }
 
@@ -1246,62 +1307,73 @@ int repack(mvs_unet *n, cudaStream_t st)
 
 inline int grid_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 16LL * kSMs); }
 
-int conv_fwd(mvs_unet *n, int l, const bf16 *in, bf16 *out, int lvl, cudaStream_t st)
+// one tensor, or the concatenation of `prev` (nearest upsampled) and `skip`
+Act act(const bf16 *p, int channels) { return Act{p, nullptr, channels, 0}; }
+Act cat(const bf16 *prev, int cp, const bf16 *skip, int cs) { return Act{prev, skip, cp + cs, cp}; }
+
+int conv_fwd(mvs_unet *n, int l, const Act &in, bf16 *out, int lvl, cudaStream_t st, const Head &head = Head{})
 {
     const ConvLayer &c = n->L[l];
-    return launch_conv(in, c.cin, c.wf, n->params + c.b_off, nullptr, out, c.cout, n->B, n->H >> lvl, n->W >> lvl, 1,
-                       n->err, st);
+    return launch_conv(in, c.wf, n->params + c.b_off, Act{}, out, c.cout, n->B, n->H >> lvl, n->W >> lvl, 1, n->err, st,
+                       head);
 }
+int conv_fwd(mvs_unet *n, int l, const bf16 *in, bf16 *out, int lvl, cudaStream_t st)
+{
+    return conv_fwd(n, l, act(in, n->L[l].cin), out, lvl, st);
+}
+
+// what the decoder levels read
+Act cat2(const mvs_unet *n) { return cat(n->e3, 128, n->e2, 64); }
+Act cat1(const mvs_unet *n) { return cat(n->d2, 64, n->e1, 32); }
+Act cat0(const mvs_unet *n) { return cat(n->d1, 32, n->e0, 16); }
 
 int forward(mvs_unet *n, const float *wta, const float *cost, const float *ref255, cudaStream_t st)
 {
     const long long npix = (long long)n->B * n->H * n->W;
-    features_kernel<<<grid_for(npix), 256, 0, st>>>(wta, cost, ref255, npix, n->nm, n->x0);
+    MVS_TRY_CUDA(launch_dependent(features_kernel, dim3(grid_for(npix)), dim3(256), 0, st, wta, cost, ref255, npix, n->nm,
+                                  n->x0));
     const int B = n->B, H = n->H, W = n->W;
-    auto pool = [&](const bf16 *in, int lvl, int C, bf16 *out) {
+    auto pool = [&](const bf16 *in, int lvl, int C, bf16 *out) -> int {
         const long long m = (long long)B * (H >> (lvl + 1)) * (W >> (lvl + 1)) * (C / 8);
-        pool_kernel<<<grid_for(m), 256, 0, st>>>(in, B, H >> lvl, W >> lvl, C, out);
-    };
-    auto upcat = [&](const bf16 *prev, int cp, const bf16 *skip, int cs, int lvl, bf16 *out) {
-        const long long m = (long long)B * (H >> lvl) * (W >> lvl) * ((cp + cs) / 8);
-        upcat_kernel<<<grid_for(m), 256, 0, st>>>(prev, cp, skip, cs, B, H >> lvl, W >> lvl, out);
+        MVS_TRY_CUDA(launch_dependent(pool_kernel, dim3(grid_for(m)), dim3(256), 0, st, in, B, H >> lvl, W >> lvl, C, out));
+        return MVS_OK;
     };
     MVS_RC(conv_fwd(n, E0A, n->x0, n->e0a, 0, st));
     MVS_RC(conv_fwd(n, E0B, n->e0a, n->e0, 0, st));
-    pool(n->e0, 0, 16, n->p0);
+    MVS_RC(pool(n->e0, 0, 16, n->p0));
     MVS_RC(conv_fwd(n, E1A, n->p0, n->e1a, 1, st));
     MVS_RC(conv_fwd(n, E1B, n->e1a, n->e1, 1, st));
-    pool(n->e1, 1, 32, n->p1);
+    MVS_RC(pool(n->e1, 1, 32, n->p1));
     MVS_RC(conv_fwd(n, E2A, n->p1, n->e2a, 2, st));
     MVS_RC(conv_fwd(n, E2B, n->e2a, n->e2, 2, st));
-    pool(n->e2, 2, 64, n->p2);
+    MVS_RC(pool(n->e2, 2, 64, n->p2));
     MVS_RC(conv_fwd(n, E3A, n->p2, n->e3a, 3, st));
     MVS_RC(conv_fwd(n, E3B, n->e3a, n->e3, 3, st));
-    upcat(n->e3, 128, n->e2, 64, 2, n->c2);
-    MVS_RC(conv_fwd(n, D2A, n->c2, n->d2a, 2, st));
+    MVS_RC(conv_fwd(n, D2A, cat2(n), n->d2a, 2, st));
     MVS_RC(conv_fwd(n, D2B, n->d2a, n->d2, 2, st));
-    upcat(n->d2, 64, n->e1, 32, 1, n->c1);
-    MVS_RC(conv_fwd(n, D1A, n->c1, n->d1a, 1, st));
+    MVS_RC(conv_fwd(n, D1A, cat1(n), n->d1a, 1, st));
     MVS_RC(conv_fwd(n, D1B, n->d1a, n->d1, 1, st));
-    upcat(n->d1, 32, n->e0, 16, 0, n->c0);
-    MVS_RC(conv_fwd(n, D0A, n->c0, n->d0a, 0, st));
-    MVS_RC(conv_fwd(n, D0B, n->d0a, n->d0, 0, st));
-    head_kernel<<<grid_for(npix), 256, 0, st>>>(n->d0, n->params + n->head_w, n->params + n->head_b, wta, npix,
-                                                (long long)H * W, n->nm, n->u, n->v);
+    MVS_RC(conv_fwd(n, D0A, cat0(n), n->d0a, 0, st));
+    const Head head{n->params + n->head_w, n->params + n->head_b, wta, n->u, n->v, n->nm};
+    MVS_RC(conv_fwd(n, D0B, act(n->d0a, 16), n->d0, 0, st, head));
     return check_launch("unet forward");
 }
 
 // backward of conv layer l: dz = gradient at its (pre-ReLU-masked) output;
 // weight/bias gradients from its input x; dx (optional) masked by x > 0 when
 // mask_x
-int conv_bwd(mvs_unet *n, int l, const bf16 *x, const bf16 *dz, bf16 *dx, bool mask_x, int lvl, cudaStream_t st)
+int conv_bwd(mvs_unet *n, int l, const Act &x, const bf16 *dz, bf16 *dx, bool mask_x, int lvl, cudaStream_t st)
 {
     const ConvLayer &c = n->L[l];
     const int H = n->H >> lvl, W = n->W >> lvl;
-    MVS_RC(launch_wgrad(x, c.cin, dz, c.cout, n->B, H, W, n->grads + c.w_off, n->grads + c.b_off, n->err, st));
+    MVS_RC(launch_wgrad(x, dz, c.cout, n->B, H, W, n->grads + c.w_off, n->grads + c.b_off, n->err, st));
     if (dx)
-        MVS_RC(launch_conv(dz, c.cout, c.wb, nullptr, mask_x ? x : nullptr, dx, c.cin, n->B, H, W, 0, n->err, st));
+        MVS_RC(launch_conv(act(dz, c.cout), c.wb, nullptr, mask_x ? x : Act{}, dx, c.cin, n->B, H, W, 0, n->err, st));
     return MVS_OK;
+}
+int conv_bwd(mvs_unet *n, int l, const bf16 *x, const bf16 *dz, bf16 *dx, bool mask_x, int lvl, cudaStream_t st)
+{
+    return conv_bwd(n, l, act(x, n->L[l].cin), dz, dx, mask_x, lvl, st);
 }
 
 int backward(mvs_unet *n, const float *ut, const float *vt, cudaStream_t st)
@@ -1313,39 +1385,44 @@ int backward(mvs_unet *n, const float *ut, const float *vt, cudaStream_t st)
     head_back_kernel<<<std::min<long long>((npix + 255) / 256, 4LL * kSMs), 256, 0, st>>>(
         n->d0, n->params + n->head_w, n->u, n->v, ut, vt, npix, (long long)H * W, n->nm, n->gd0,
         n->grads + n->head_w, n->grads + n->head_b, n->loss);
-    auto upback = [&](const bf16 *dc, int ctot, int lvl, int cp, bf16 *dprev) {
+    auto upback = [&](const bf16 *dc, int ctot, int lvl, int cp, bf16 *dprev) -> int {
         const long long m = (long long)B * (H >> (lvl + 1)) * (W >> (lvl + 1)) * (cp / 8);
-        upcat_back_kernel<<<grid_for(m), 256, 0, st>>>(dc, ctot, B, H >> lvl, W >> lvl, cp, dprev);
+        MVS_TRY_CUDA(launch_dependent(upcat_back_kernel, dim3(grid_for(m)), dim3(256), 0, st, dc, ctot, B, H >> lvl,
+                                      W >> lvl, cp, dprev));
+        return MVS_OK;
     };
-    auto poolback = [&](const bf16 *dp, const bf16 *dc, int ctot, int coff, const bf16 *e, int lvl, int C, bf16 *de) {
+    auto poolback = [&](const bf16 *dp, const bf16 *dc, int ctot, int coff, const bf16 *e, int lvl, int C,
+                        bf16 *de) -> int {
         const long long m = (long long)B * (H >> lvl) * (W >> lvl) * (C / 8);
-        pool_back_kernel<<<grid_for(m), 256, 0, st>>>(dp, dc, ctot, coff, e, B, H >> lvl, W >> lvl, C, de);
+        MVS_TRY_CUDA(launch_dependent(pool_back_kernel, dim3(grid_for(m)), dim3(256), 0, st, dp, dc, ctot, coff, e, B,
+                                      H >> lvl, W >> lvl, C, de));
+        return MVS_OK;
     };
     // decoder level 0
     MVS_RC(conv_bwd(n, D0B, n->d0a, n->gd0, n->gd0a, true, 0, st));
-    MVS_RC(conv_bwd(n, D0A, n->c0, n->gd0a, n->gc0, true, 0, st));
-    upback(n->gc0, 48, 0, 32, n->gd1);
+    MVS_RC(conv_bwd(n, D0A, cat0(n), n->gd0a, n->gc0, true, 0, st));
+    MVS_RC(upback(n->gc0, 48, 0, 32, n->gd1));
     // decoder level 1
     MVS_RC(conv_bwd(n, D1B, n->d1a, n->gd1, n->gd1a, true, 1, st));
-    MVS_RC(conv_bwd(n, D1A, n->c1, n->gd1a, n->gc1, true, 1, st));
-    upback(n->gc1, 96, 1, 64, n->gd2);
+    MVS_RC(conv_bwd(n, D1A, cat1(n), n->gd1a, n->gc1, true, 1, st));
+    MVS_RC(upback(n->gc1, 96, 1, 64, n->gd2));
     // decoder level 2
     MVS_RC(conv_bwd(n, D2B, n->d2a, n->gd2, n->gd2a, true, 2, st));
-    MVS_RC(conv_bwd(n, D2A, n->c2, n->gd2a, n->gc2, true, 2, st));
-    upback(n->gc2, 192, 2, 128, n->ge3);
+    MVS_RC(conv_bwd(n, D2A, cat2(n), n->gd2a, n->gc2, true, 2, st));
+    MVS_RC(upback(n->gc2, 192, 2, 128, n->ge3));
     // bottleneck
     MVS_RC(conv_bwd(n, E3B, n->e3a, n->ge3, n->ge3a, true, 3, st));
     MVS_RC(conv_bwd(n, E3A, n->p2, n->ge3a, n->gp2, false, 3, st));
     // encoder level 2
-    poolback(n->gp2, n->gc2, 192, 128, n->e2, 2, 64, n->ge2);
+    MVS_RC(poolback(n->gp2, n->gc2, 192, 128, n->e2, 2, 64, n->ge2));
     MVS_RC(conv_bwd(n, E2B, n->e2a, n->ge2, n->ge2a, true, 2, st));
     MVS_RC(conv_bwd(n, E2A, n->p1, n->ge2a, n->gp1, false, 2, st));
     // encoder level 1
-    poolback(n->gp1, n->gc1, 96, 64, n->e1, 1, 32, n->ge1);
+    MVS_RC(poolback(n->gp1, n->gc1, 96, 64, n->e1, 1, 32, n->ge1));
     MVS_RC(conv_bwd(n, E1B, n->e1a, n->ge1, n->ge1a, true, 1, st));
     MVS_RC(conv_bwd(n, E1A, n->p0, n->ge1a, n->gp0, false, 1, st));
     // encoder level 0
-    poolback(n->gp0, n->gc0, 48, 32, n->e0, 0, 16, n->ge0);
+    MVS_RC(poolback(n->gp0, n->gc0, 48, 32, n->e0, 0, 16, n->ge0));
     MVS_RC(conv_bwd(n, E0B, n->e0a, n->ge0, n->ge0a, true, 0, st));
     MVS_RC(conv_bwd(n, E0A, n->x0, n->ge0a, nullptr, false, 0, st));
     return check_launch("unet backward");
@@ -1508,8 +1585,8 @@ int mvs_conv3x3_forward(const uint16_t *d_in, int32_t cin, const float *d_w, con
 {
     if (!d_in || !d_w || !d_out || !d_wpack || !d_err) return set_error(MVS_ERR_ARG, "null argument");
     cudaStream_t st = (cudaStream_t)stream;
-    pack_kernel<<<ceil_div(9 * cin * cout, 256), 256, 0, st>>>(d_w, cin, cout, d_wpack, nullptr);
-    MVS_RC(launch_conv(d_in, cin, d_wpack, d_bias, nullptr, d_out, cout, batch, height, width, relu, d_err, st));
+    MVS_RC(launch_pack(d_w, cin, cout, d_wpack, nullptr, st));
+    MVS_RC(launch_conv(act(d_in, cin), d_wpack, d_bias, Act{}, d_out, cout, batch, height, width, relu, d_err, st));
     return check_launch("conv3x3 forward");
 }
 
@@ -1521,11 +1598,11 @@ int mvs_conv3x3_backward(const uint16_t *d_x, int32_t cin, const float *d_w, con
     if (cout % 16 || cin % 16) return set_error(MVS_ERR_ARG, "channels must be multiples of 16");
     cudaStream_t st = (cudaStream_t)stream;
     const size_t s = (size_t)9 * cin * cout;
-    pack_kernel<<<ceil_div((int)s, 256), 256, 0, st>>>(d_w, cin, cout, d_wpack, d_wpack + s);
-    MVS_RC(launch_wgrad(d_x, cin, d_dz, cout, batch, height, width, d_dw, d_db, d_err, st, tensor_cores != 0));
+    MVS_RC(launch_pack(d_w, cin, cout, d_wpack, d_wpack + s, st));
+    MVS_RC(launch_wgrad(act(d_x, cin), d_dz, cout, batch, height, width, d_dw, d_db, d_err, st, tensor_cores != 0));
     if (d_dx)
-        MVS_RC(launch_conv(d_dz, cout, d_wpack + s, nullptr, mask_x ? d_x : nullptr, d_dx, cin, batch, height, width,
-                           0, d_err, st));
+        MVS_RC(launch_conv(act(d_dz, cout), d_wpack + s, nullptr, mask_x ? act(d_x, cin) : Act{}, d_dx, cin, batch,
+                           height, width, 0, d_err, st));
     return check_launch("conv3x3 backward");
 }
 
