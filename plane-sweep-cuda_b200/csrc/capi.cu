@@ -33,7 +33,7 @@ int check_launch(const char *what)
 void clear_error() { g_err[0] = 0; }
 
 // sweep.cu
-int sweep_pick_chunks(int win, int w, int h, int V, int P, int mode);
+int sweep_pick_chunks(int win, int w, int h, int V, int P, int mode, int moments);
 int sweep_launch(const mvs_sweep_desc *d, const float *ref, const float *srcs, const float *H, const float *depths,
                  float *depth, int32_t *labels, float *best, uint16_t *cost, unsigned long long *scratch,
                  int n_chunks, void *stream, float4 *quad = nullptr);
@@ -223,7 +223,8 @@ int mvs_sweep(const mvs_sweep_desc *d, const float *ref, const float *srcs, cons
         return set_error(MVS_ERR_ARG, "workspace of %zu bytes needed, %zu given", need, ws ? ws_bytes : (size_t)0);
     if (((uintptr_t)ws) & 7) return set_error(MVS_ERR_ARG, "workspace must be 8-byte aligned");
     if (d->mode == MVS_SWEEP_PER_VIEW && cost) return set_error(MVS_ERR_ARG, "cost volume is an aggregated-mode output");
-    const int chunks = sweep_pick_chunks(d->window, d->width, d->height, d->n_views, d->n_planes, d->mode);
+    const int chunks = sweep_pick_chunks(d->window, d->width, d->height, d->n_views, d->n_planes, d->mode,
+                                         d->moments);
     float4 *quad = (float4 *)((char *)ws + (sweep_scratch_bytes(d) + 255) / 256 * 256);
     return sweep_launch(d, ref, srcs, H, depths, depth, labels, best, cost, (unsigned long long *)ws, chunks, stream,
                         quad);

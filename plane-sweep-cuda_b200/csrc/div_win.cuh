@@ -24,4 +24,50 @@ __device__ __forceinline__ float div_win(float x)
     return isfinite(x) && x != 0.f ? __fmaf_rn(r, y, q) : q;
 }
 
+// Two floats in a register pair, for the packed FP32 instructions (each half
+// rounds as the scalar instruction does).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 p, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// div_win of both halves
+template <int WIN>
+__device__ __forceinline__ void div_win2(f32x2 x, float &oa, float &ob)
+{
+    constexpr float d = (float)WIN, y = 1.f / (float)WIN;
+    const f32x2 yy = pack2(y, y), q = mul2(x, yy), z = fma2(fma2(q, pack2(-d, -d), x), yy, q);
+    float xa, xb, qa, qb, za, zb;
+    unpack2(x, xa, xb);
+    unpack2(q, qa, qb);
+    unpack2(z, za, zb);
+    oa = isfinite(xa) && xa != 0.f ? za : qa;
+    ob = isfinite(xb) && xb != 0.f ? zb : qb;
+}
+
 }  // namespace mvs

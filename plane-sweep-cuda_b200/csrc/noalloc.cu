@@ -23,7 +23,7 @@
 
 namespace mvs {
 
-int sweep_pick_chunks(int win, int w, int h, int V, int P, int mode);
+int sweep_pick_chunks(int win, int w, int h, int V, int P, int mode, int moments);
 int sweep_launch(const mvs_sweep_desc *d, const float *ref, const float *srcs, const float *H, const float *depths,
                  float *depth, int32_t *labels, float *best, uint16_t *cost, unsigned long long *scratch,
                  int n_chunks, void *stream, float4 *quad);
@@ -61,7 +61,8 @@ int mvs_sweep_noalloc(const mvs_sweep_desc *d, const float *ref, const float *sr
     const cudaError_t e = cudaGetSymbolAddress(&scratch, g_sweep_scratch);
     if (e != cudaSuccess)
         return set_error(MVS_ERR_CUDA, "cudaGetSymbolAddress(sweep scratch): %s", cudaGetErrorString(e));
-    const int chunks = sweep_pick_chunks(d->window, d->width, d->height, d->n_views, d->n_planes, d->mode);
+    const int chunks = sweep_pick_chunks(d->window, d->width, d->height, d->n_views, d->n_planes, d->mode,
+                                         d->moments);
     return sweep_launch(d, ref, srcs, H, depths, depth, labels, best, cost, (unsigned long long *)scratch, chunks,
                         stream, nullptr);
 }

@@ -43,6 +43,7 @@
 
 #include "common.cuh"
 #include "div_win.cuh"
+#include "quot.cuh"
 
 namespace mvs {
 namespace {
@@ -163,6 +164,58 @@ __device__ __forceinline__ void row_sums(const float (*CSq)[CSP], float *out)
             out[j] = m;
         }
     }
+}
+
+// The reference arithmetic's column sums of w and w^2 lie side by side, so that
+// pass A1 and pass B add both in one packed instruction (the sums are added
+// term by term, in window order, and are two thirds of that mode's additions).
+// The pairs' row pitch of 148 floats, 20 (mod 32), spreads the 8 rows of a
+// quarter warp's 16-byte loads over all banks.
+constexpr int CSP2 = 74;
+static_assert(CSP2 <= CSP && CSP2 >= RWMAX + 2 && CSP2 % 2 == 0, "pairs fit the two arrays they replace");
+typedef float2 (*PairRows)[CSP2];
+__device__ __forceinline__ PairRows pair_rows(float (*CS)[TH][CSP]) { return reinterpret_cast<PairRows>(&CS[0][0][0]); }
+
+template <int WIN, int TWS = 0>
+__device__ __forceinline__ void row_sums_pairs(const float2 (*C)[CSP2], float *o1, float *o2)
+{
+    using G = Geo<WIN, TWS>;
+    constexpr int NV = G::RUN + 2 * G::R;
+    static_assert(7 * G::RUN + (NV + 1) / 2 * 2 <= CSP2, "run loads stay inside a row");
+    f32x2 v[NV + 1];
+    const float2 *row = C[b_row()] + b_seg() * G::RUN;
+    if constexpr (G::RUN % 2 == 0) {
+        const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(row);
+#pragma unroll
+        for (int i = 0; i < (NV + 1) / 2; ++i) {
+            const ulonglong2 t = q[i];
+            v[2 * i] = t.x;
+            v[2 * i + 1] = t.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = reinterpret_cast<const f32x2 *>(row)[i];
+    }
+#pragma unroll
+    for (int j = 0; j < G::RUN; ++j) {
+        f32x2 m = 0ull;
+#pragma unroll
+        for (int i = 0; i < WIN; ++i) m = add2(m, v[j + i]);
+        div_win2<WIN>(m, o1[j], o2[j]);
+    }
+}
+
+// Row sums of pass B: w, w^2 and ref * w.
+template <int WIN, int MOM, int TWS = 0>
+__device__ __forceinline__ void row_sums3(float (*CS)[TH][CSP], float *s1, float *s2, float *s12)
+{
+    if constexpr (MOM == MVS_MOMENTS_REFERENCE) {
+        row_sums_pairs<WIN, TWS>(pair_rows(CS), s1, s2);
+    } else {
+        row_sums<WIN, MOM, TWS>(CS[0], s1);
+        row_sums<WIN, MOM, TWS>(CS[1], s2);
+    }
+    row_sums<WIN, MOM, TWS>(CS[2], s12);
 }
 
 // Rounding bound of n*Sxx - Sx^2 for the compensated sums, as a multiple of
@@ -421,9 +474,13 @@ constexpr int kFloorMagicBits = 0x4B400000;
 // pass A0 with the row coordinates from shared memory; with QUAD, `quad` holds
 // the source's 2x2 neighbourhoods (difference form in COMPENSATED), else the
 // four samples are gathered from `src`.  COMPENSATED stores the samples
-// shifted by `shift`.
-template <int WIN, int MOM, bool QUAD, int TWS = 0, bool ROWS_INTERIOR = false>
-__device__ __forceinline__ void pass_a0_rows(float (*Wt)[RWMAX], const float *__restrict__ src,
+// shifted by `shift`.  QUICK: the reference's divisions by quotients().  CLAMP:
+// samples outside the source load its first word instead of nothing, which
+// saves clearing their registers (measured faster in the reference arithmetic,
+// by 0.5 to 1%, and in the batched kernel, by 4%, and 2% slower in the single-frame
+// compensated kernel).
+template <int WIN, int MOM, bool QUAD, int TWS, bool ROWS_INTERIOR, bool QUICK, bool CLAMP>
+__device__ __forceinline__ void a0_rows(float (*Wt)[RWMAX], const float *__restrict__ src,
                                              const float4 *__restrict__ quad, int w, int h, const float *Hm, float X,
                                              const float *Yc, float shift)
 {
@@ -457,8 +514,15 @@ __device__ __forceinline__ void pass_a0_rows(float (*Wt)[RWMAX], const float *__
                     const float q0 = Hm[0] * X + Hm[1] * Y + Hm[2] * 1.f;
                     const float q1 = Hm[3] * X + Hm[4] * Y + Hm[5] * 1.f;
                     const float q2 = Hm[6] * X + Hm[7] * Y + Hm[8] * 1.f;
-                    xs = q0 / q2 - 1.f;
-                    ys = q1 / q2 - 1.f;
+                    float qx, qy;
+                    if (QUICK) {
+                        quotients(q0, q1, q2, qx, qy);
+                    } else {
+                        qx = q0 / q2;
+                        qy = q1 / q2;
+                    }
+                    xs = qx - 1.f;
+                    ys = qy - 1.f;
                 } else {
                     const float q0 = fmaf(Hm[1], Y, a0), q1 = fmaf(Hm[4], Y, a1), q2 = fmaf(Hm[7], Y, a2);
                     float rz;
@@ -479,8 +543,8 @@ __device__ __forceinline__ void pass_a0_rows(float (*Wt)[RWMAX], const float *__
 #pragma unroll
             for (int j = 0; j < BATCH; ++j) {
                 d00[j] = d01[j] = d10[j] = d11[j] = 0.f;
-                if (ok[j]) {
-                    const float4 q = __ldg(quad + off[j]);
+                if (CLAMP || ok[j]) {
+                    const float4 q = __ldg(quad + (!CLAMP || ok[j] ? off[j] : 0u));
                     d00[j] = q.x;
                     d01[j] = q.y;
                     d10[j] = q.z;
@@ -522,6 +586,28 @@ __device__ __forceinline__ void pass_a0_rows(float (*Wt)[RWMAX], const float *__
     }
 }
 
+// Pass A0.  The reference's homographies are normalised to H22 = 1, so a depth q2
+// is 0 or at least 2^-25 in magnitude (a sum with 1 of floats whose exponents are
+// not below its own by more than 24 places), and with the entries beside it below
+// 2^60 quotients() gives its divisions: where a coordinate may lie inside the
+// source it is the correctly rounded one, elsewhere both forms lie outside.  Other
+// homographies keep the IEEE divisions.  (640x480, 8 views, 256 planes, 9x9, per
+// view: 5.44 -> 5.15 ms with this, the packed sums and the clamped loads.)
+template <int WIN, int MOM, bool QUAD, int TWS = 0, bool ROWS_INTERIOR = false, bool CLAMP = false>
+__device__ __forceinline__ void pass_a0_rows(float (*Wt)[RWMAX], const float *__restrict__ src,
+                                             const float4 *__restrict__ quad, int w, int h, const float *Hm, float X,
+                                             const float *Yc, float shift)
+{
+    if constexpr (MOM == MVS_MOMENTS_REFERENCE) {
+        if (Hm[8] == 1.f && fabsf(Hm[6]) < 0x1p60f && fabsf(Hm[7]) < 0x1p60f)
+            a0_rows<WIN, MOM, QUAD, TWS, ROWS_INTERIOR, true, true>(Wt, src, quad, w, h, Hm, X, Yc, shift);
+        else
+            a0_rows<WIN, MOM, QUAD, TWS, ROWS_INTERIOR, false, true>(Wt, src, quad, w, h, Hm, X, Yc, shift);
+    } else {
+        a0_rows<WIN, MOM, QUAD, TWS, ROWS_INTERIOR, false, CLAMP>(Wt, src, quad, w, h, Hm, X, Yc, shift);
+    }
+}
+
 // pass A1 with the reference column read from shared memory: thread (c, s)
 // forms the column sums of w, w^2 and ref*w for output rows [11 s, 11 s + 11)
 // (COMPENSATED: Wt and Rf hold shifted values already)
@@ -541,19 +627,17 @@ __device__ __forceinline__ void pass_a1_rows(const float (*Wt)[RWMAX], float (*C
 #pragma unroll
         for (int k = 0; k < STRIP; ++k) {
             if (k == STRIP - 1 && !full) break;
-            float s1 = 0.f, s2 = 0.f, s12 = 0.f;
+            float s1, s2, s12 = 0.f;
+            f32x2 ss = 0ull;
 #pragma unroll
             for (int i = 0; i < WIN; ++i) {
                 const float x = wv[k + i];
-                s1 = s1 + x;
-                s2 = s2 + x * x;
+                ss = add2(ss, pack2(x, x * x));
                 s12 = s12 + Rf[r0 + k + i][c] * x;
             }
-            s1 = div_win<WIN>(s1);
-            s2 = div_win<WIN>(s2);
+            div_win2<WIN>(ss, s1, s2);
             s12 = div_win<WIN>(s12);
-            CS[0][r0 + k][c] = s1;
-            CS[1][r0 + k][c] = s2;
+            pair_rows(CS)[r0 + k][c] = make_float2(s1, s2);
             CS[2][r0 + k][c] = s12;
         }
     } else {
@@ -649,10 +733,11 @@ __device__ __forceinline__ void aggregated_tile(AggSmem &A, const SweepArgs &a, 
             float hn = 0.f;
             if (threadIdx.x < 9 && np < p1) hn = ldg(a.H + ((size_t)nv * a.P + np) * 9 + threadIdx.x);
             if (a.quad && rows_interior)
-                pass_a0_rows<WIN, MOM, true, TWS, true>(S.Wt, nullptr, a.quad + (size_t)view * n, w, h, Hm, Xcol, A.Yc,
+                pass_a0_rows<WIN, MOM, true, TWS, true, BATCHED>(S.Wt, nullptr, a.quad + (size_t)view * n, w, h, Hm, Xcol, A.Yc,
                                                         sh);
             else if (a.quad)
-                pass_a0_rows<WIN, MOM, true, TWS>(S.Wt, nullptr, a.quad + (size_t)view * n, w, h, Hm, Xcol, A.Yc, sh);
+                pass_a0_rows<WIN, MOM, true, TWS, false, BATCHED>(S.Wt, nullptr, a.quad + (size_t)view * n, w, h, Hm, Xcol,
+                                                              A.Yc, sh);
             else
                 pass_a0_rows<WIN, MOM, false, TWS>(S.Wt, a.srcs + (size_t)view * n, nullptr, w, h, Hm, Xcol, A.Yc, sh);
             if (threadIdx.x < 9) S.Hm[hb ^ 1][threadIdx.x] = hn;
@@ -661,9 +746,7 @@ __device__ __forceinline__ void aggregated_tile(AggSmem &A, const SweepArgs &a, 
             pass_a1_rows<WIN, MOM, TWS>(S.Wt, S.CS, A.Rf);
             __syncthreads();
             float s1[G::RUN], s2[G::RUN], s12[G::RUN];
-            row_sums<WIN, MOM, TWS>(S.CS[0], s1);
-            row_sums<WIN, MOM, TWS>(S.CS[1], s2);
-            row_sums<WIN, MOM, TWS>(S.CS[2], s12);
+            row_sums3<WIN, MOM, TWS>(S.CS, s1, s2, s12);
             ncc_run<WIN, MOM, TWS>(s1, s2, s12, A.RM[ly] + lx, A.RS[ly] + lx, a.stdthresh,
                               [&](int j, float c) { acc[j] += c; });
         }
@@ -770,9 +853,7 @@ __global__ void __launch_bounds__(THREADS, 3) sweep_view_kernel(SweepArgs a)
         pass_a1_rows<WIN, MOM>(S.Wt, S.CS, A.Rf);
         __syncthreads();
         float s1[G::RUN], s2[G::RUN], s12[G::RUN];
-        row_sums<WIN, MOM>(S.CS[0], s1);
-        row_sums<WIN, MOM>(S.CS[1], s2);
-        row_sums<WIN, MOM>(S.CS[2], s12);
+        row_sums3<WIN, MOM>(S.CS, s1, s2, s12);
         ncc_run<WIN, MOM, 0>(s1, s2, s12, A.RM[ly] + lx, A.RS[ly] + lx, a.stdthresh, [&](int j, float c) {
             if (c > best[j]) {
                 best[j] = c;
@@ -1061,9 +1142,7 @@ __global__ void __launch_bounds__(THREADS, 2) sweep_aggregated_tma_kernel(SweepA
             pass_a1_rows<WIN, MOM>(S.Wt, S.CS, A.Rf);
             __syncthreads();
             float s1[G::RUN], s2[G::RUN], s12[G::RUN];
-            row_sums<WIN, MOM>(S.CS[0], s1);
-            row_sums<WIN, MOM>(S.CS[1], s2);
-            row_sums<WIN, MOM>(S.CS[2], s12);
+            row_sums3<WIN, MOM>(S.CS, s1, s2, s12);
             ncc_run<WIN, MOM, 0>(s1, s2, s12, A.RM[ly] + lx, A.RS[ly] + lx, a.stdthresh,
                                  [&](int j, float c) { acc[j] += c; });
         }
@@ -1477,29 +1556,30 @@ int tiles_for(int win, int w, int h)
 }  // namespace
 
 // Plane chunking.  A CTA costs its planes plus a start-up (reference moments,
-// merging its winners) worth about 1.5 planes per view, 4 planes of one view
-// when it walks all of them.  Up to three CTAs share an SM: m = 1, 2, 3 of them
-// take 0.6, 0.87 and 1.22 times what one takes at full occupancy, and x waves of
-// three about x + 0.5 (the last wave is partly empty).  The planes per CTA with
-// the smallest product are taken, within 2% (once 7%) of the fastest one tried on
-// the B200 (eleven cases, 160x120 to 1242x375, 1 to 8 views, 37 to 256 planes).
+// merging its winners) worth about 1.5 planes per view in the reference
+// arithmetic, 3 in the compensated one, and 4 planes of one view when it walks all
+// of them.  Up to three CTAs share an SM: m = 1, 2, 3 of them take 0.6, 0.9 and
+// 1.22 times what one takes at full occupancy, and x waves of three about x + 0.5
+// (the last wave is partly empty).  The planes per CTA with the smallest product
+// are taken, within 2% of the fastest one tried on the B200 (twelve cases,
+// 160x120 to 1242x375, 1 to 8 views, 37 to 256 planes).
 // Against a fixed target of 8 CTAs per SM with 16 planes at least: 320x240, 4
 // views, 64 planes, 7x7, aggregated 208 -> 120 us (one full wave instead of a
 // third of one), per view 233 -> 217 us; 640x480, 8 views, 256 planes, 9x9,
 // aggregated 2.98 -> 2.75 ms, per view 5.98 -> 5.43 ms.  (The merge of chunks is
 // exact, so the results do not depend on it.)
-int sweep_pick_chunks(int win, int w, int h, int V, int P, int mode)
+int sweep_pick_chunks(int win, int w, int h, int V, int P, int mode, int moments)
 {
     const bool per_view = mode == MVS_SWEEP_PER_VIEW;
     const double tiles = (double)tiles_for(win, w, h) * (per_view ? V : 1);
-    const double start = per_view ? 1.5 : 4.0 / V;
+    const double start = !per_view ? 4.0 / V : moments == MVS_MOMENTS_REFERENCE ? 1.5 : 3.0;
     int best = 1;
     double cost = 1e300;
     for (int planes = P; planes >= 1; planes = planes > 64 ? planes - planes / 16 : planes - 1) {
         const int chunks = ceil_div(P, planes);
         if ((per_view ? (long)chunks * V : chunks) > 65535) break;   // the grid's z extent
         const double m = ceil(tiles * chunks / kSMs), x = tiles * chunks / (3.0 * kSMs);
-        const double c = (planes + start) * (m <= 1 ? 0.6 : m <= 2 ? 0.87 : m <= 3 ? 1.22 : x + 0.5);
+        const double c = (planes + start) * (m <= 1 ? 0.6 : m <= 2 ? 0.9 : m <= 3 ? 1.22 : x + 0.5);
         if (c < cost) {
             cost = c;
             best = chunks;
