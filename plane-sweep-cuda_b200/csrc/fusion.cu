@@ -247,21 +247,25 @@ __device__ __forceinline__ void p_step(float px, float py, float pz, float vi, f
     }
 }
 
-// Slices per thread of the U and P steps: their loads are all in flight at once,
-// and a slice's z neighbour is the thread's own next (or last) one.  Both steps
-// are bound by HBM (68 bytes per voxel and iteration, 93% of the measured copy
-// rate); 256^3 x 200 iterations: 40.6 ms with one slice per thread, 37.7 ms with
-// two (1.5% of it from P's order below), 37.4 ms with four, which cost the small
-// volumes more (100 x 77 x 61, 10 bins, 50 iterations: 0.48 against 0.51 ms).
-constexpr int ZB = 2;
-
-template <int BINS>
+// ZB slices per thread of the U and P steps: their loads are all in flight at
+// once, and a slice's z neighbour is the thread's own next (or last) one.  Large
+// volumes are bound by HBM (68 bytes per voxel and iteration, 93% of the measured
+// copy rate); 256^3 x 200 iterations: 40.6 ms with one slice per thread, 37.7 ms
+// with two (1.5% of it from P's order below), 37.4 ms with four.  Two slices halve
+// the CTAs, and a grid below two waves then ends on a few of them: see
+// slices_per_thread().
+//
+// The next step's launch is allowed after the loads with two slices (the next
+// CTAs start while these compute and store), and at the end with one: with the
+// whole grid resident, CTAs let in early fill the free places unevenly and the
+// next step runs as long as the fullest SM (49 x 83 x 52, 7.1 us an iteration let
+// in at the start, 6.8 us at the end).
+template <int BINS, int ZB>
 __global__ void __launch_bounds__(VX *VY) update_u_kernel(Dims D, const uint16_t *__restrict__ hist,
                                                          float *__restrict__ u, float *__restrict__ v,
                                                          const float *__restrict__ p, double tau, double lambda)
 {
     wait_for_previous_grid();   // launched as a dependent launch: the previous step is complete
-    allow_next_grid();
     constexpr int HS = HistStride<BINS>::value;
     const int x = blockIdx.x * VX + threadIdx.x, y = blockIdx.y * VY + threadIdx.y, z0 = blockIdx.z * ZB;
     if (x >= D.vw || y >= D.vh) return;
@@ -288,6 +292,7 @@ __global__ void __launch_bounds__(VX *VY) update_u_kernel(Dims D, const uint16_t
 #pragma unroll
         for (int e = 0; e < HS / 8; ++e) c[k][e] = __ldcs(h4 + e);
     }
+    if (ZB > 1) allow_next_grid();
 #pragma unroll
     for (int k = 0; k < ZB; ++k) {
         if (z0 + k >= D.vd) break;
@@ -302,16 +307,17 @@ __global__ void __launch_bounds__(VX *VY) update_u_kernel(Dims D, const uint16_t
         u[i0 + k * sz] = un;
         v[i0 + k * sz] = vn;
     }
+    if (ZB == 1) allow_next_grid();
 }
 
 // The slabs run from the last to the first: the U step ended there, so the p and
 // v that it left in L2 are read before they are displaced, and the next U step
 // starts where this one ended.
+template <int ZB>
 __global__ void __launch_bounds__(VX *VY) update_p_kernel(Dims D, const float *__restrict__ v, float *__restrict__ p,
                                                          float sigma)
 {
     wait_for_previous_grid();   // launched as a dependent launch: the previous step is complete
-    allow_next_grid();
     const int x = blockIdx.x * VX + threadIdx.x, y = blockIdx.y * VY + threadIdx.y;
     const int z0 = (gridDim.z - 1 - blockIdx.z) * ZB;
     if (x >= D.vw || y >= D.vh) return;
@@ -334,6 +340,7 @@ __global__ void __launch_bounds__(VX *VY) update_p_kernel(Dims D, const float *_
         ay[k] = py[o];
         az[k] = pz[o];
     }
+    if (ZB > 1) allow_next_grid();
 #pragma unroll
     for (int k = 0; k < ZB; ++k) {
         if (z0 + k >= D.vd) break;
@@ -343,6 +350,7 @@ __global__ void __launch_bounds__(VX *VY) update_p_kernel(Dims D, const float *_
         py[k * sz] = qy;
         pz[k * sz] = qz;
     }
+    if (ZB == 1) allow_next_grid();
 }
 
 __global__ void extract_count_kernel(const float *__restrict__ u, long n, float lo, float hi,
@@ -414,8 +422,19 @@ Dims dims_of(int vw, int vh, int vd, const float *a, const float *b)
 
 const float kZero3[3] = {0.f, 0.f, 0.f};
 
-dim3 slab_grid(int vw, int vh, int vd) { return dim3((vw + VX - 1) / VX, (vh + VY - 1) / VY, (vd + ZB - 1) / ZB); }
-dim3 voxel_grid(int vw, int vh, int vd) { return dim3((vw + VX - 1) / VX, (vh + VY - 1) / VY, vd); }
+dim3 slab_grid(int vw, int vh, int vd, int zb = 1)
+{
+    return dim3((vw + VX - 1) / VX, (vh + VY - 1) / VY, (vd + zb - 1) / zb);
+}
+
+// Two slices per thread from two waves of one-slice CTAs on (8 per SM).  Against
+// one slice, 30 volumes of 33 to 256 voxels a side: 1.02-1.13x from two waves on
+// (256^3 1.06x, 161 x 63 x 215 1.13x, 100 x 77 x 61 1.03x), 0.77-1.03x below.
+int slices_per_thread(int vw, int vh, int vd)
+{
+    const dim3 g = slab_grid(vw, vh, vd);
+    return (size_t)g.x * g.y * g.z >= 2 * 8 * 148 ? 2 : 1;
+}
 
 }  // namespace
 
@@ -428,7 +447,7 @@ int fusion_histogram(int vw, int vh, int vd, int bins, const float *a, const flo
 {
     const Dims D = dims_of(vw, vh, vd, a, b);
     switch (bins) {
-#define H(N) case N: histogram_kernel<N><<<voxel_grid(vw, vh, vd), dim3(VX, VY), 0, st>>>(D, hist, depths, w, h, nmaps, d_cams, thr); break;
+#define H(N) case N: histogram_kernel<N><<<slab_grid(vw, vh, vd), dim3(VX, VY), 0, st>>>(D, hist, depths, w, h, nmaps, d_cams, thr); break;
         MVS_BINS(H)
 #undef H
     default: return set_error(MVS_ERR_ARG, "bins %d not supported (2..10)", bins);
@@ -440,8 +459,9 @@ int fusion_update_u(int vw, int vh, int vd, int bins, const uint16_t *hist, floa
                     double tau, double lambda, cudaStream_t st)
 {
     const Dims D = dims_of(vw, vh, vd, kZero3, kZero3);
+    const int zb = slices_per_thread(vw, vh, vd);
     switch (bins) {
-#define U(N) case N: MVS_TRY_CUDA(launch_dependent(update_u_kernel<N>, slab_grid(vw, vh, vd), dim3(VX, VY), 0, st, D, hist, u, v, p, tau, lambda)); break;
+#define U(N) case N: MVS_TRY_CUDA(launch_dependent(zb == 2 ? update_u_kernel<N, 2> : update_u_kernel<N, 1>, slab_grid(vw, vh, vd, zb), dim3(VX, VY), 0, st, D, hist, u, v, p, tau, lambda)); break;
         MVS_BINS(U)
 #undef U
     default: return set_error(MVS_ERR_ARG, "bins %d not supported (2..10)", bins);
@@ -452,7 +472,9 @@ int fusion_update_u(int vw, int vh, int vd, int bins, const uint16_t *hist, floa
 int fusion_update_p(int vw, int vh, int vd, const float *v, float *p, double sigma, cudaStream_t st)
 {
     const Dims D = dims_of(vw, vh, vd, kZero3, kZero3);
-    MVS_TRY_CUDA(launch_dependent(update_p_kernel, slab_grid(vw, vh, vd), dim3(VX, VY), 0, st, D, v, p, (float)sigma));
+    const int zb = slices_per_thread(vw, vh, vd);
+    MVS_TRY_CUDA(launch_dependent(zb == 2 ? update_p_kernel<2> : update_p_kernel<1>, slab_grid(vw, vh, vd, zb),
+                                  dim3(VX, VY), 0, st, D, v, p, (float)sigma));
     return check_launch("fusion update_p_kernel");
 }
 

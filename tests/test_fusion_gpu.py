@@ -98,6 +98,30 @@ def test_prox_median_matches_insertion_sort(cuda, bins, top):
     np.testing.assert_array_equal(r["u"], prox_want(hist, u0, bins, tau, lam))
 
 
+# a grid of 32 x 8 x 1 blocks takes two slices per thread from 2368 blocks on: one block row less,
+# an odd depth just above it (half a slab at the end), and volumes that fill no block
+@pytest.mark.parametrize("bins", [2, 3, 8, 9, 10])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (32, 8, 3), (65, 3, 5), (33, 9, 591), (33, 9, 593), (31, 17, 790)])
+def test_iterations_at_slab_edges_bit_exact_vs_oracle(cuda, dims, bins):
+    rng = np.random.default_rng(11)
+    n = dims[0] * dims[1] * dims[2]
+    hist = rng.integers(0, 6, size=(bins, n)).astype(np.uint16)
+    u0 = rng.uniform(-1.5, 1.5, n).astype(np.float32)
+    p0 = rng.uniform(-0.8, 0.8, (3, n)).astype(np.float32)
+    vol = M.FusionVolume(dims, bins, [0, 0, 0], [1, 1, 1])
+    vol.upload(u=u0, v=u0, p=p0, hist=hist)
+    vol.tvl1(3, 0.1, 0.5, 1.0)
+    r = vol.download()
+    vol.close()
+    o = po.Volume(bins, dims, [0, 0, 0], [1, 1, 1], precision="f32")
+    o.u[:], o.v[:], o.p[:], o.hist[:] = u0, u0, p0, hist
+    for _ in range(3):
+        o.update_u(0.1, 0.5)
+        o.update_p(1.0)
+    for k in ("u", "v", "p"):
+        np.testing.assert_array_equal(r[k], getattr(o, k))
+
+
 class _DeviceArray:
     """A device pointer of the library as an array that torch can wrap without a copy."""
 
