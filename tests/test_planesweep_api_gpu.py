@@ -59,6 +59,32 @@ def test_run_algorithm_bit_exact(cuda, golden, name, from_list):
         ps.getDepthmap(out=np.empty((3, 3), np.float32))
 
 
+@pytest.mark.parametrize("step", ["denoise", "tgv", "sparse"])
+def test_refined_8bit_maps_and_new_reference(cuda, golden, step):
+    """The 8-bit map of each refinement is ConvertDepthtoUChar of its float map, here with the
+    depths partly outside znear..zfar, and a reference image set after the sweep is the one used."""
+    g = golden("sweep_refloop_w7")
+    ps = make_ps(g, False)
+    ps.RunAlgorithm()
+    ps.set_reference(np.ascontiguousarray(g["ref"][::-1]), g["Rref"], g["tref"])
+    d = g["depth"]
+    lo, hi = np.float32(np.quantile(d, 0.2)), np.float32(np.quantile(d, 0.8))
+    ps.setZ(lo, hi)
+    if step == "denoise":
+        ps.CudaDenoise(niters=7)
+        m, m8 = ps.getDepthmapDenoised(), ps.getDepthmap8uDenoised()
+        want = po.tvl1_denoise(g["ref"][::-1], d, float(lo), float(hi), niters=7, precision="f32")
+        np.testing.assert_array_equal(m, want)
+    elif step == "tgv":
+        ps.TGV(niters=3, warps=2)
+        m, m8 = ps.getDepthmapTGV(), ps.getDepthmap8uTGV()
+    else:
+        ps.TGVdenoiseFromSparse(np.where(d > lo, d, 0).astype(np.float32), 5)
+        m, m8 = ps.getDepthmapTGV(), ps.getDepthmap8uTGV()
+    c = np.clip((m - lo) / (hi - lo), np.float32(0), np.float32(1))
+    np.testing.assert_array_equal(m8, np.where(m == m, (np.float32(255) * c).astype(np.uint8), 255).astype(np.uint8))
+
+
 def test_denoise_tgv_and_points_follow_the_reference(cuda, golden):
     g = golden("sweep_refloop_w7")
     ps = make_ps(g, False)
