@@ -477,15 +477,15 @@ int launch_conv(const Act &in, const bf16 *wpack, const float *bias, const Act &
 // ---------------------------------------------------------------------------
 // weight gradient on tensor cores: for every tap (ky, kx),
 //   D[co][kx][ky][ci] += sum_p dz[p][co] * x[p + (ky, kx)][ci]
-// with K = pixels, for 16-channel chunks of the input.  A = dz^T (M = 64 or 128
-// output channels) is MN-major, [co / 8][pixel][8].  B is the tile's input halo
-// itself, stored so that one descriptor reaches three taps: rows of 10 pixels x
-// 16 bytes ordered [halo row][8-channel group], so the (ky, group) neighbour of
-// a core matrix (8 pixels of a tile row x 8 channels) lies 160 bytes further
-// for each step of 2 ky + group, the next tile row 320 bytes further, and tap
-// kx starts 16 kx bytes later.  A K-step of 16 pixels (two tile rows) is then
-// three MMAs with N = 3 ky x 16 channels = 48, straight from the bytes that
-// cp.async brought: nothing is expanded or copied in shared memory.
+// with K = pixels, for chunks of NC = 16, 32 or 48 input channels (G = NC / 8
+// groups).  A = dz^T (M = 64 or 128 output channels) is MN-major, [co / 8][pixel][8].
+// B is the tile's input halo itself, stored so that one descriptor reaches three
+// taps: rows of 10 pixels x 16 bytes ordered [halo row][8-channel group], so the
+// (ky, group) neighbour of a core matrix (8 pixels of a tile row x 8 channels) lies
+// 160 bytes further for each step of G ky + group, the next tile row 160 G bytes
+// further, and tap kx starts 16 kx bytes later.  A K-step of 16 pixels (two tile
+// rows) is then three MMAs with N = 3 ky x NC channels, straight from the bytes
+// that cp.async brought: nothing is expanded or copied in shared memory.
 // ---------------------------------------------------------------------------
 
 struct WgArgs {
@@ -498,10 +498,9 @@ struct WgArgs {
 };
 
 constexpr int WG_COPY = 256, WG_TC_THREADS = WG_COPY + 32;   // eight copying warps and one that issues the MMAs
-constexpr int WG_NC = 16;                                      // input channels per chunk
+constexpr int WG_NC = 16;                                      // input channels of a chunk, or 2 or 3 times as many
 constexpr int WG_HALO_W = TW + 2, WG_HALO_H = TH + 2;          // 10 x 18 input pixels around an 8 x 16 tile
-constexpr int WG_HALO_BYTES = 2 * WG_HALO_H * WG_HALO_W * 16;  // 5760
-constexpr int WG_N = 3 * WG_NC;                                // columns of one MMA: (ky, channel)
+constexpr int WG_HALO_BYTES = 2 * WG_HALO_H * WG_HALO_W * 16;  // 5760 per 16 channels
 constexpr int WG_SMEM_SM = 228 * 1024;   // shared memory of an SM, 1 KB of it reserved per CTA
 constexpr int WG_MAX_STAGES = 8;
 // tiles a CTA sums at least: each adds its 9 x 16 x cout sums to dW atomically
@@ -515,11 +514,11 @@ struct WgLayout {
     int a_bytes, stage_bytes, bytes;
 };
 
-__host__ __device__ inline WgLayout wg_layout(int m, int stages, int cg)
+__host__ __device__ inline WgLayout wg_layout(int m, int stages, int cg, int nc)
 {
     WgLayout L;
     L.a_bytes = cg * 128 * 16;
-    L.stage_bytes = L.a_bytes + WG_HALO_BYTES;
+    L.stage_bytes = L.a_bytes + nc / WG_NC * WG_HALO_BYTES;
     L.bytes = stages * L.stage_bytes + (m / 8) * 128 * 16 + 128;
     return L;
 }
@@ -544,25 +543,29 @@ __device__ __forceinline__ void red_add4(float *dst, float a, float b, float c, 
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// A CTA sums a run of 8 x 16 tiles for one 16-channel chunk of the input
+// A CTA sums a run of 8 x 16 tiles for one chunk of NC input channels
 // (blockIdx.y) and one block of M output channels (blockIdx.z) in tensor memory:
 // a ring of R stages is filled by cp.async R - 1 tiles ahead, one thread issues
 // the 24 MMAs of a tile, and tcgen05.commit on the stage's mbarrier frees it.
 // Every wait is bounded.  M = 64 keeps rows 16 q .. 16 q + 15 of the accumulator
 // in lanes 32 q .. 32 q + 15.
 //
-// What bounds it: shared-memory reads of the MMAs (3.5 KB each at M = 64, 24 per
-// tile and chunk) and, on the inner levels, the latency of few tiles per CTA.
-template <int M, int R>
+// What bounds it: shared-memory reads of the MMAs (24 per tile and chunk, each 2 KB
+// of dz at M = 64, of which 16 output channels use a quarter, and 0.1 KB per input
+// channel; 48 input channels take 115 cycles an MMA, 16 take 65) and, on the inner
+// levels, the latency of few tiles per CTA.
+template <int M, int R, int NC>
 __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
 {
     static_assert(R >= 2 && R <= WG_MAX_STAGES, "at least two stages");
-    constexpr int TMEM_COLS = 256;   // 3 WG_N = 144 used
+    constexpr int SUB = NC / WG_NC, G = NC / 8;   // 16-channel parts, 8-channel groups
+    constexpr int N = 3 * NC;                     // columns of one MMA: (ky, channel)
+    constexpr int TMEM_COLS = 3 * N <= 256 ? 256 : 512;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ci0 = blockIdx.y * WG_NC, co0 = blockIdx.z * M;
+    const int ci0 = blockIdx.y * NC, co0 = blockIdx.z * M;
     const int cg = min(a.cout - co0, M) >> 3;
-    const WgLayout L = wg_layout(M, R, cg);
+    const WgLayout L = wg_layout(M, R, cg, NC);
     uint64_t *bars = (uint64_t *)(smem + L.bytes - 128);
     uint32_t *tmem_slot = (uint32_t *)(smem + L.bytes - 128 + 8 * WG_MAX_STAGES);
     const int t_begin = blockIdx.x * a.tiles_per_cta;
@@ -599,14 +602,18 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
         const int pix = k >> 1, g = k & 1, y = pix / WG_HALO_W, x = pix - y * WG_HALO_W;
         h_y[i] = y - 1;
         h_x[i] = x - 1;
-        h_dst[i] = k < HALO_ITEMS ? ((y * 2 + g) * WG_HALO_W + x) * 16 : -1;
+        h_dst[i] = k < HALO_ITEMS ? ((y * G + g) * WG_HALO_W + x) * 16 : -1;
     }
-    const Source sx = act_source(a.x, ci0);
-    int h_off[HI];
+    Source sx[SUB];
+    int h_off[SUB][HI];
 #pragma unroll
-    for (int i = 0; i < HI; ++i) h_off[i] = source_delta(sx, W, h_y[i], h_x[i]);
+    for (int q = 0; q < SUB; ++q) {
+        sx[q] = act_source(a.x, ci0 + q * WG_NC);
+        sx[q].p += 8 * (tid & 1);
+#pragma unroll
+        for (int i = 0; i < HI; ++i) h_off[q][i] = source_delta(sx[q], W, h_y[i], h_x[i]);
+    }
     const int dz_off = (dz_y * W + dz_x) * cout;
-    const bf16 *xg = sx.p + 8 * (tid & 1);
     const bf16 *zg = a.dz + co0 + 8 * dz_g0;
     // the next tile to copy: image lb, tile row and column lty, ltx
     const int per_img = a.tiles_x * a.tiles_y;
@@ -617,22 +624,31 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
         const int y0 = lty * TH, x0 = ltx * TW;
         const uint32_t ab = sbase + s * L.stage_bytes, hb = ab + L.a_bytes;
         const size_t pb = (size_t)lb * img + (size_t)y0 * W + x0;
-        const bf16 *zt = zg + pb * cout + dz_off, *xt = xg + source_at(sx, H, W, lb, y0, x0);
+        const bf16 *zt = zg + pb * cout + dz_off;
         uint32_t zd = ab + (dz_g0 * 128 + dz_m) * 16;
         if (y0 > 0 && x0 > 0 && y0 + TH < H && x0 + TW < W) {   // halo and all inside the image
             for (int g = dz_g0; g < cg; g += 2, zt += 16, zd += 2 * 128 * 16) cp_async16(zd, zt, true);
 #pragma unroll
-            for (int i = 0; i < HI; ++i)
-                if (h_dst[i] >= 0) cp_async16(hb + h_dst[i], xt + h_off[i], true);
+            for (int q = 0; q < SUB; ++q) {
+                const bf16 *xt = sx[q].p + source_at(sx[q], H, W, lb, y0, x0);
+#pragma unroll
+                for (int i = 0; i < HI; ++i)
+                    if (h_dst[i] >= 0) cp_async16(hb + h_dst[i] + q * 2 * WG_HALO_W * 16, xt + h_off[q][i], true);
+            }
         } else {
             const bool ok = y0 + dz_y < H && x0 + dz_x < W;
             if (!ok) zt = a.dz;
             for (int g = dz_g0; g < cg; g += 2, zt += ok ? 16 : 0, zd += 2 * 128 * 16) cp_async16(zd, zt, ok);
 #pragma unroll
-            for (int i = 0; i < HI; ++i) {
-                const int gy = y0 + h_y[i], gx = x0 + h_x[i];
-                const bool in = gy >= 0 && gy < H && gx >= 0 && gx < W;
-                if (h_dst[i] >= 0) cp_async16(hb + h_dst[i], in ? xt + h_off[i] : a.x.p, in);
+            for (int q = 0; q < SUB; ++q) {
+                const bf16 *xt = sx[q].p + source_at(sx[q], H, W, lb, y0, x0);
+#pragma unroll
+                for (int i = 0; i < HI; ++i) {
+                    const int gy = y0 + h_y[i], gx = x0 + h_x[i];
+                    const bool in = gy >= 0 && gy < H && gx >= 0 && gx < W;
+                    if (h_dst[i] >= 0)
+                        cp_async16(hb + h_dst[i] + q * 2 * WG_HALO_W * 16, in ? xt + h_off[q][i] : a.x.p, in);
+                }
             }
         }
         cp_async_commit();
@@ -642,7 +658,7 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
         }
     };
 
-    constexpr uint32_t idesc = idesc_bf16_mn(M, WG_N);
+    constexpr uint32_t idesc = idesc_bf16_mn(M, N);
     const int n = t_end - t_begin;
     bool failed = false;
     int last = -1;   // the last tile whose MMAs were issued (the same in every thread)
@@ -661,12 +677,12 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
             tc_fence_after();
             // descriptors differ only in their start address (16-byte units)
             const uint32_t ab = sbase + (c % R) * L.stage_bytes, hb = ab + L.a_bytes;
-            const uint64_t ad = smem_desc(ab, 128, 128 * 16), bd = smem_desc(hb, 2 * WG_HALO_W * 16, WG_HALO_W * 16);
+            const uint64_t ad = smem_desc(ab, 128, 128 * 16), bd = smem_desc(hb, G * WG_HALO_W * 16, WG_HALO_W * 16);
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
                 for (int kx = 0; kx < 3; ++kx)
-                    mma_bf16(tmem + kx * WG_N, ad + 16 * ks, bd + 4 * ks * WG_HALO_W + kx, idesc,
+                    mma_bf16(tmem + kx * N, ad + 16 * ks, bd + 2 * G * ks * WG_HALO_W + kx, idesc,
                              (c > 0 || ks > 0) ? 1u : 0u);
             mma_commit(&bars[c % R]);
         }
@@ -706,11 +722,11 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
         const bool own = (M == 128 || lane < 16) && co0 + row < cout;
         float *dst = a.dW + ((size_t)(co0 + row) * cin + ci0) * 9;
 #pragma unroll 1
-        for (int cq = warp >> 2; cq < WG_NC / 4 && copies; cq += 2) {
+        for (int cq = warp >> 2; cq < NC / 4 && copies; cq += 2) {
             float v[9][4];
 #pragma unroll
             for (int t = 0; t < 9; ++t)
-                tmem_ld4(tmem + ((uint32_t)(quarter * 32) << 16) + (t % 3) * WG_N + (t / 3) * WG_NC + 4 * cq, v[t]);
+                tmem_ld4(tmem + ((uint32_t)(quarter * 32) << 16) + (t % 3) * N + (t / 3) * NC + 4 * cq, v[t]);
             tmem_ld_wait();
             if (!own) continue;
             if (a.vec) {
@@ -732,17 +748,17 @@ __global__ void __launch_bounds__(WG_TC_THREADS) wgrad_tc_kernel(WgArgs a)
     }
 }
 
-// One launch in one wave of two CTAs per SM: the CTAs of every (chunk, output
-// block) split the tiles evenly (a last wave of a few CTAs would cost a whole
-// run of tiles), with at least WG_MIN_TILES each.
-template <int M, int R>
+// One launch in one wave: the CTAs of every (chunk, output block) split the tiles
+// evenly (a last wave of a few CTAs would cost a whole run of tiles), with at
+// least WG_MIN_TILES each.
+template <int M, int R, int NC>
 int launch_wgrad_tc_t(WgArgs a, cudaStream_t st)
 {
-    const WgLayout L = wg_layout(M, R, std::min(a.cout, M) >> 3);
-    const int chunks = a.cin / WG_NC, coblocks = ceil_div(a.cout, M);
-    const int xctas = std::max(1, 2 * kSMs / (chunks * coblocks));
+    const WgLayout L = wg_layout(M, R, std::min(a.cout, M) >> 3, NC);
+    const int chunks = a.cin / NC, coblocks = ceil_div(a.cout, M);
+    const int xctas = std::max(1, (NC == WG_NC ? 2 : 1) * kSMs / (chunks * coblocks));
     a.tiles_per_cta = std::max(ceil_div(a.n_tiles, xctas), WG_MIN_TILES);
-    auto kernel = wgrad_tc_kernel<M, R>;
+    auto kernel = wgrad_tc_kernel<M, R, NC>;
     MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L.bytes));
     MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                       (int)cudaSharedmemCarveoutMaxShared));
@@ -751,20 +767,22 @@ int launch_wgrad_tc_t(WgArgs a, cudaStream_t st)
     return MVS_OK;
 }
 
-// The deepest ring of which two CTAs fit an SM.
-template <int M>
+// The deepest ring of which two CTAs (one with wide chunks, whose sums take all of
+// the tensor memory) fit an SM.
+template <int M, int NC>
 int launch_wgrad_tc_m(const WgArgs &a, cudaStream_t st)
 {
+    const int room = (NC == WG_NC ? WG_SMEM_SM / 2 : WG_SMEM_SM) - 1024;
     int r = WG_MAX_STAGES;
-    while (r > 2 && wg_layout(M, r, std::min(a.cout, M) >> 3).bytes > WG_SMEM_SM / 2 - 1024) --r;
+    while (r > 2 && wg_layout(M, r, std::min(a.cout, M) >> 3, NC).bytes > room) --r;
     switch (r) {
-    case 8: return launch_wgrad_tc_t<M, 8>(a, st);
-    case 7: return launch_wgrad_tc_t<M, 7>(a, st);
-    case 6: return launch_wgrad_tc_t<M, 6>(a, st);
-    case 5: return launch_wgrad_tc_t<M, 5>(a, st);
-    case 4: return launch_wgrad_tc_t<M, 4>(a, st);
-    case 3: return launch_wgrad_tc_t<M, 3>(a, st);
-    default: return launch_wgrad_tc_t<M, 2>(a, st);
+    case 8: return launch_wgrad_tc_t<M, 8, NC>(a, st);
+    case 7: return launch_wgrad_tc_t<M, 7, NC>(a, st);
+    case 6: return launch_wgrad_tc_t<M, 6, NC>(a, st);
+    case 5: return launch_wgrad_tc_t<M, 5, NC>(a, st);
+    case 4: return launch_wgrad_tc_t<M, 4, NC>(a, st);
+    case 3: return launch_wgrad_tc_t<M, 3, NC>(a, st);
+    default: return launch_wgrad_tc_t<M, 2, NC>(a, st);
     }
 }
 
@@ -774,7 +792,21 @@ int launch_wgrad_tc(const Act &x, const bf16 *dz, int cout, int B, int H, int W,
     if (cout % 8 || cin % WG_NC) return set_error(MVS_ERR_ARG, "wgrad: cin %d, cout %d", cin, cout);
     WgArgs a{x, dz, dW, err, B, H, W, cin, cout, ceil_div(W, TW), ceil_div(H, TH), 1, 0, ((uintptr_t)dW & 15) == 0};
     a.n_tiles = B * a.tiles_x * a.tiles_y;
-    return cout <= 64 ? launch_wgrad_tc_m<64>(a, st) : launch_wgrad_tc_m<128>(a, st);
+    // Wide chunks read dz once for 48 or 32 input channels and issue a third or half of
+    // the MMAs, but leave one CTA per SM: only where the runs of WG_MIN_TILES tiles
+    // still make a CTA for every SM (4 x 640 x 480, 48 -> 16 channels: 130 us in chunks
+    // of 16, 93 of 48; 32 -> 32: 34 and 31; a training step of it 2025 and 1937 us, of
+    // 2 x 320 x 240 940 and 907; below that size the rule keeps 16 nearly everywhere).
+    const int coblocks = cout <= 64 ? 1 : ceil_div(cout, 128);
+    auto fills = [&](int nc) {
+        return cin % nc == 0 && a.n_tiles / WG_MIN_TILES * (cin / nc) * coblocks >= kSMs;
+    };
+    const int nc = fills(3 * WG_NC) ? 3 * WG_NC : fills(2 * WG_NC) ? 2 * WG_NC : WG_NC;
+    if (nc == 3 * WG_NC)
+        return cout <= 64 ? launch_wgrad_tc_m<64, 3 * WG_NC>(a, st) : launch_wgrad_tc_m<128, 3 * WG_NC>(a, st);
+    if (nc == 2 * WG_NC)
+        return cout <= 64 ? launch_wgrad_tc_m<64, 2 * WG_NC>(a, st) : launch_wgrad_tc_m<128, 2 * WG_NC>(a, st);
+    return cout <= 64 ? launch_wgrad_tc_m<64, WG_NC>(a, st) : launch_wgrad_tc_m<128, WG_NC>(a, st);
 }
 
 // ---------------------------------------------------------------------------

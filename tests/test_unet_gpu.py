@@ -76,6 +76,55 @@ def test_conv3x3_forward_and_backward(cuda, cin, cout):
     assert _rel(dw2.cpu().numpy().reshape(cout, cin, 9), rdw) < 1e-5
 
 
+# chunks of 48 and 32 input channels are taken from 148 runs of 8 tiles (8 x 16 pixels) on: sizes
+# just there, with ragged tiles, for 64 and 128 rows of output channels
+@pytest.mark.parametrize("cin,cout,H,W", [(48, 16, 511, 293), (32, 16, 505, 296), (32, 48, 300, 500), (96, 32, 300, 250),
+                                          (64, 128, 300, 250), (192, 128, 157, 240)])
+def test_weight_gradient_in_wide_chunks(cuda, cin, cout, H, W):
+    import torch
+    import mvs_b200 as M
+    rng = np.random.default_rng(cin + cout)
+    x = torch.from_numpy(np.maximum(rng.normal(size=(1, H, W, cin)), -0.2).astype(np.float32)).to(cuda)
+    dz = torch.from_numpy(rng.normal(size=(1, H, W, cout)).astype(np.float32)).to(cuda)
+    x, dz = x.to(torch.bfloat16).contiguous(), dz.to(torch.bfloat16).contiguous()
+    w = torch.zeros((cout, cin, 3, 3), device=cuda)
+    dw = torch.zeros((cout, cin, 3, 3), device=cuda)
+    wpack = torch.empty(2 * 9 * cin * cout, dtype=torch.bfloat16, device=cuda)
+    err = torch.zeros(1, dtype=torch.int32, device=cuda)
+    M.conv3x3_backward(x, w, dz, False, None, dw, None, wpack, err)
+    assert int(err.item()) == 0
+    xp = torch.nn.functional.pad(x[0].double(), (0, 0, 1, 1, 1, 1))
+    z = dz[0].double().reshape(-1, cout)
+    want = torch.stack([z.T @ xp[ky:ky + H, kx:kx + W].reshape(-1, cin) for ky in range(3) for kx in range(3)], -1)
+    # at most 64 sums of a tile's K steps and 148 atomic adds, each within 2^-23 of the sum so far
+    assert _rel(dw.cpu().numpy().reshape(cout, cin, 9), want.cpu().numpy()) < (64 + 148) * 2.0 ** -23
+
+
+def test_gradients_of_a_repeated_frame(cuda):
+    """A batch of one frame twice has the frame's gradients (its pixels weigh exactly half as much):
+    the first decoder level's then come from chunks of 48 channels of the concatenation, the single
+    frame's from chunks of 16.  Only the order of FP32 sums differs; a wrong channel gives O(1)."""
+    import torch
+    import mvs_b200 as M
+    H, W = 240, 320
+    rng = np.random.default_rng(6)
+    inputs = _net_inputs(rng, 1, H, W)
+    grads = []
+    for B in (1, 2):
+        net = M.Unet(B, H, W)
+        net.init_params(seed=4)
+        a = [torch.from_numpy(np.ascontiguousarray(np.repeat(t, B, 0))).to(cuda) for t in inputs]
+        net.forward(*a[:3])
+        net.backward(*a[3:])
+        net.check()
+        grads.append(net.get_params(grads=True)[1])
+        layers = [net.layer_info(l) for l in range(14)]
+    for l, (ci, co, wo, bo) in enumerate(layers):
+        n = 9 * ci * co
+        assert np.linalg.norm(grads[0][wo:wo + n]) > 0
+        assert _rel(grads[1][wo:wo + n], grads[0][wo:wo + n]) < 1e-3, l
+
+
 def _net_inputs(rng, B, H, W):
     """Random inputs; targets offset coherently from the input depth so that the
     gradients are sums without heavy cancellation."""
