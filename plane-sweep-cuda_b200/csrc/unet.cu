@@ -22,8 +22,9 @@
 // stores bf16.
 //
 // The backward pass w.r.t. the input is the same kernel with the weights
-// flipped and transposed; the weight gradient is a per-tap reduction over
-// pixels on the CUDA cores (FP32), with the bias gradient.
+// flipped and transposed.  The weight gradient is a second tensor-core kernel
+// with K = pixels (and a per-tap reduction on the CUDA cores that it is tested
+// against), the bias gradient a reduction over pixels.
 #include <math.h>
 #include <string.h>
 
