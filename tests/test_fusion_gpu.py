@@ -122,6 +122,28 @@ def test_iterations_at_slab_edges_bit_exact_vs_oracle(cuda, dims, bins):
         np.testing.assert_array_equal(r[k], getattr(o, k))
 
 
+def test_dual_step_with_infinities_and_nan(cuda):
+    """Sums of squares at 1, just past 1, infinite and NaN in the dual step, against the f32 oracle."""
+    rng = np.random.default_rng(4)
+    dims, bins = (33, 9, 7), 7
+    n = 33 * 9 * 7
+    p0 = rng.uniform(-1.2, 1.2, (3, n)).astype(np.float32)
+    p0[:, 10:200] *= 1e19
+    p0[:, 210:260] = 0
+    p0[0, 210:230] = np.nextafter(np.float32(1), np.float32(2)) - np.arange(20, dtype=np.float32) * 2.0 ** -24
+    p0[0, 300], p0[1, 310], p0[2, 320] = np.inf, np.nan, -np.inf
+    v0 = np.where(np.arange(n) < 400, 0, rng.uniform(-1, 1, n)).astype(np.float32)
+    vol = M.FusionVolume(dims, bins, [0, 0, 0], [1, 1, 1])
+    vol.upload(v=v0, p=p0)
+    vol.update_p(1.0)
+    r = vol.download()
+    o = po.Volume(bins, dims, [0, 0, 0], [1, 1, 1], precision="f32")
+    o.v[:], o.p[:] = v0, p0
+    o.update_p(1.0)
+    assert np.isnan(r["p"]).any()
+    np.testing.assert_array_equal(r["p"], o.p)
+
+
 class _DeviceArray:
     """A device pointer of the library as an array that torch can wrap without a copy."""
 
