@@ -106,6 +106,18 @@ __device__ __forceinline__ float bf2f(uint16_t b) { return __uint_as_float((uint
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+constexpr size_t kSmemMax = 227 * 1024;   // shared memory of a CTA
+
+// Lets a kernel be launched with up to `most` bytes of dynamic shared memory.  That
+// limit is a setting of the process, and a launch above it is refused: calls on
+// other threads may set it between this call and its launches, so `most` is the
+// kernel's maximum over all sizes, the same in every call.
+template <typename K>
+cudaError_t allow_shared_memory(K *kernel, size_t most)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // Programmatic dependent launch, for loops of short dependent launches (one
 // launch per iteration).  A kernel launched with launch_dependent() may be
 // scheduled while the previous kernel of its stream is still finishing, which

@@ -650,7 +650,6 @@ struct BlockBufs {
 };
 
 constexpr int TGW = 12;   // warps per CTA at most
-constexpr size_t kSmemMax = 227 * 1024;   // shared memory of a CTA
 // shared memory per warp: T11, T12, T22, u0, u, u1x, u1y and the views' r, It, Iu
 // of each cell, and the rows exchanged with its neighbours
 constexpr size_t block_warp_bytes(int V)
@@ -1761,7 +1760,7 @@ int tgv2_sparse_run(int w, int h, const float *ref255, const float *depthmap, co
     // 320x240: 475 us with 6 and 12; 1242x375: 1.40 ms with 4 and 20)
     const BlockPlan plan = block_plan(w, h, niters, SPW, 6.5, 0.11);
     const size_t smem = kSparseWarpBytes * plan.warps;
-    MVS_TRY_CUDA(cudaFuncSetAttribute(sparse_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MVS_TRY_CUDA(allow_shared_memory(sparse_block_kernel, kSparseWarpBytes * SPW));
     for (int it = 0; it < niters; it += b.iters) {
         b.iters = min(plan.iters, niters - it);
         b.halo = block_halo(b.iters);
@@ -1984,7 +1983,7 @@ int tgv2_run(int w, int h, int V, const float *ref255, const float *srcs255, con
     }
     if (blocked) {
         bsmem = block_warp_bytes(V) * plan.warps + kBlockBytes;
-        MVS_TRY_CUDA(cudaFuncSetAttribute(block_kernel(V), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
+        MVS_TRY_CUDA(allow_shared_memory(block_kernel(V), kSmemMax));
         bb.ctl = ib.ctl;
         bb.T11 = L.T11;
         bb.T12 = L.T12;

@@ -81,6 +81,7 @@ struct Bufs {
 // an iteration at 640x480, of which the IEEE double square root and divisions
 // of the projections were a third; 3.0 us in this form (B200).
 constexpr int BW = kBlockW, RPT = kBlockRows, MAXWARPS = 32;
+constexpr size_t kWarpBytes = (size_t)3 * RPT * 32 * sizeof(double2);   // dynamic shared memory per warp: the tensor
 
 template <bool THETA1>
 __global__ void __launch_bounds__(32 * MAXWARPS) tvl1_block_kernel(Bufs b)
@@ -289,9 +290,9 @@ int tvl1_run(int w, int h, const float *ref255, float *depth, float znear, float
     // per 100 iterations, against 324 us for 4 and 14 and 389 us for 2 and 24;
     // 320x240: 6 and 12, 176 us; 1242x375: 400 us)
     const BlockPlan plan = block_plan(w, h, prm->niters, MAXWARPS, 4.2, 0.08);
-    const size_t smem = (size_t)3 * RPT * plan.warps * 32 * sizeof(double2);
+    const size_t smem = kWarpBytes * plan.warps;
     auto kernel = b.theta == 1.f ? tvl1_block_kernel<true> : tvl1_block_kernel<false>;
-    MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MVS_TRY_CUDA(allow_shared_memory(kernel, kWarpBytes * MAXWARPS));
     for (int it = 0; it < prm->niters; it += b.iters) {
         b.iters = min(plan.iters, prm->niters - it);
         b.halo = block_halo(b.iters);
