@@ -435,7 +435,7 @@ int launch_conv_n(const ConvArgs &a, int B, cudaStream_t st)
 {
     using S = ConvSmem<COUT, MT>;
     auto kernel = conv3x3_tc_kernel<COUT, MT, NST>;
-    MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::bytes(NST)));
+    MVS_TRY_CUDA(allow_shared_memory(kernel, S::bytes(NST)));
     MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                       (int)cudaSharedmemCarveoutMaxShared));
     const int tiles = a.tiles_x * ceil_div(a.H, MT * TH);
@@ -451,7 +451,7 @@ int launch_conv_n(const ConvArgs &a, int B, cudaStream_t st)
 template <int COUT, int MT = 1>
 int launch_conv_t(const ConvArgs &a, int B, cudaStream_t st)
 {
-    static_assert(ConvSmem<COUT, MT>::bytes(3) <= 227 * 1024, "three stages fit a CTA");
+    static_assert(ConvSmem<COUT, MT>::bytes(3) <= kSmemMax, "three stages fit a CTA");
     if (a.cin <= 16) return launch_conv_n<COUT, MT, 1>(a, B, st);
     if (a.cin <= 32) return launch_conv_n<COUT, MT, 2>(a, B, st);
     return launch_conv_n<COUT, MT, 3>(a, B, st);
@@ -760,7 +760,8 @@ int launch_wgrad_tc_t(WgArgs a, cudaStream_t st)
     const int xctas = std::max(1, (NC == WG_NC ? 2 : 1) * kSMs / (chunks * coblocks));
     a.tiles_per_cta = std::max(ceil_div(a.n_tiles, xctas), WG_MIN_TILES);
     auto kernel = wgrad_tc_kernel<M, R, NC>;
-    MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L.bytes));
+    // (one kernel serves several counts of output channels, whose rings differ in size)
+    MVS_TRY_CUDA(allow_shared_memory(kernel, kSmemMax));
     MVS_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                       (int)cudaSharedmemCarveoutMaxShared));
     MVS_TRY_CUDA(launch_dependent(kernel, dim3(ceil_div(a.n_tiles, a.tiles_per_cta), chunks, coblocks),

@@ -28,10 +28,20 @@ for V in (1, 2, 3, 4, 5, 8, 9, 12, 13, 16):
 """,
 }
 
+NETWORK = {
+    "wgrad_tc_kernel": """
+for cin in (16, 32, 48, 64, 96, 192):
+    for cout in (16, 32, 48, 64, 96, 128, 192):
+        for h, w in ((20, 12), (480, 640)):
+            M.check(L.mvs_conv3x3_backward(ptr, cin, ptr, ptr, cout, 4, h, w, 0, None, ptr, None, ptr, ptr, 1, None))
+""",
+}
+CALLS = {**SOLVERS, **NETWORK}
 
-@pytest.mark.parametrize("kernel", SOLVERS)
+
+@pytest.mark.parametrize("kernel", CALLS)
 def test_one_shared_memory_limit_for_all_sizes(kernel):
-    log = run(SOLVERS[kernel])
+    log = run(CALLS[kernel])
     limits, seen = shared_memory_limits(log, kernel), launches(log, kernel)
     sizes = {}
     for name, _, _, smem in seen:
