@@ -2022,8 +2022,7 @@ int tgv2_run(int w, int h, int V, const float *ref255, const float *srcs255, con
             psmem = persist_smem_bytes(pth, V);
             ptiles = ceil_div(w, PT_TW) * ceil_div(h, pth);
             int per_sm = 0;
-            if (cudaFuncSetAttribute(tgv2_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)psmem) != cudaSuccess ||
+            if (allow_shared_memory(tgv2_persistent_kernel, limit) != cudaSuccess ||
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tgv2_persistent_kernel, PT_THREADS, psmem) !=
                     cudaSuccess ||
                 per_sm * sms < ptiles)

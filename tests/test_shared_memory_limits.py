@@ -26,6 +26,12 @@ for V in (1, 2, 3, 4, 5, 8, 9, 12, 13, 16):
         p = M.tgv2_params(niters=100, warps=1)
         M.check(L.mvs_tgv2_run(w, h, V, ptr, ptr, f9, f9, f9, f9, C.byref(p), 1, 1.0, ptr, None, None, ptr, big, None))
 """,
+    "tgv2_persistent_kernel": """
+f9 = (C.c_float * 144)(*[1, 0, 0, 0, 1, 0, 0, 0, 1] * 16)
+for w, h, V in ((640, 480, 8), (600, 420, 3), (320, 240, 4)):
+    p = M.tgv2_params(niters=20, warps=1, iteration_kernel=M.TGV2_ITER_PERSISTENT)
+    M.check(L.mvs_tgv2_run(w, h, V, ptr, ptr, f9, f9, f9, f9, C.byref(p), 1, 1.0, ptr, None, None, ptr, big, None))
+""",
 }
 
 NETWORK = {
