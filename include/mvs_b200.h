@@ -329,8 +329,10 @@ int mvs_ps_set_alternative_relative_matrix_method(mvs_planesweep *ps, int32_t al
 int mvs_ps_set_plane_depths(mvs_planesweep *ps, const float *depths, int32_t n);
 int mvs_ps_set_sweep_options(mvs_planesweep *ps, int32_t moments, int32_t mode, int32_t fp64_homographies);
 int mvs_ps_run_algorithm(mvs_planesweep *ps);                      /* RunAlgorithm */
+/* CudaDenoise: of the last sweep's depthmap; MVS_ERR_STATE when the reference
+ * image has been set to another size since. */
 int mvs_ps_cuda_denoise(mvs_planesweep *ps, int32_t niters, double lambda, double tau, double sigma,
-                        double theta, double beta, double gamma);  /* CudaDenoise */
+                        double theta, double beta, double gamma);
 int mvs_ps_tgv(mvs_planesweep *ps, int32_t niters, int32_t warps, double lambda, double alpha0, double alpha1,
                double tau, double sigma, double beta, double gamma); /* TGV (u = 1 start) */
 /* TGVdenoiseFromSparse: TGV2 from the last sweep depthmap towards h_sparse

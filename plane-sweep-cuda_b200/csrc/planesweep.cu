@@ -560,6 +560,11 @@ bool PlaneSweep::CudaDenoise(int, char **, const unsigned int niters, const doub
     }
     const int w = (int)depthmap.width(), h = (int)depthmap.height();
     const size_t n = (size_t)w * h;
+    if ((int)HostRef.width() != w || (int)HostRef.height() != h) {
+        mvs::set_error(MVS_ERR_STATE, "CudaDenoise: the depthmap is %dx%d, the reference image now %zux%zu: run again", w,
+                       h, HostRef.width(), HostRef.height());
+        return false;
+    }
     // A handle's images and sweep result are on the device as its setters and
     // RunAlgorithm left them; a C++ caller may have changed the host's.
     const bool on_device =

@@ -7,6 +7,7 @@
  *   copy <bytes> <kind>
  * A kernel is named as the compiler registers it (mangled). */
 #include <cuda_runtime_api.h>
+#include <pthread.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -24,11 +25,14 @@ void fake_reset(void) { text[used = 0] = 0; }
 
 static void note(const char *fmt, ...)
 {
+    static pthread_mutex_t lock = PTHREAD_MUTEX_INITIALIZER;   /* the library's copies run on several threads */
     va_list ap;
     va_start(ap, fmt);
+    pthread_mutex_lock(&lock);
     const int n = vsnprintf(text + used, sizeof(text) - used, fmt, ap);
-    va_end(ap);
     if (n > 0 && used + (size_t)n < sizeof(text)) used += (size_t)n;
+    pthread_mutex_unlock(&lock);
+    va_end(ap);
 }
 static const char *name_of(const void *f)
 {
