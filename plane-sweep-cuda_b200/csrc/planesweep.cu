@@ -618,7 +618,18 @@ bool PlaneSweep::TGVext(const mvs_tgv2_params &prm, int start, const CamImage<fl
         mvs::set_error(MVS_ERR_ARG, "TGV start depthmap missing or of the wrong size");
         return false;
     }
+    if (start == 1 && ((int)depthmap.width() != w || (int)depthmap.height() != h)) {
+        mvs::set_error(MVS_ERR_STATE, "TGV: the depthmap is %zux%zu, the reference image now %dx%d: run again",
+                       depthmap.width(), depthmap.height(), w, h);
+        return false;
+    }
     const int nimgs = std::min(std::max((int)numberimages, 1), (int)HostSrc.size());
+    for (int v = 0; v < nimgs; ++v)
+        if ((int)HostSrc[v].width() != w || (int)HostSrc[v].height() != h) {
+            mvs::set_error(MVS_ERR_STATE, "TGV: source %d is %zux%zu, reference %dx%d", v, HostSrc[v].width(),
+                           HostSrc[v].height(), w, h);
+            return false;
+        }
     depthmapTGV.reset(w, h);
     depthmap8uTGV.reset(w, h);
     if (I.ref.ensure(n * 4) || I.tvsrc.ensure(n * 4 * nimgs) || I.tvu.ensure(n * 4) || I.depth8.ensure(n) ||

@@ -49,3 +49,21 @@ refused(lambda: ps.CudaDenoise(niters=4))
 ps.set_reference(images(64, 48, 1)[0], I, zero)   # the sweep's size again
 ps.CudaDenoise(niters=4)
 """)
+
+
+@pytest.mark.parametrize("w,h", [(32, 24), (128, 96), (48, 64)])
+def test_tgv_refuses_images_of_another_size(w, h):
+    run(SETUP + f"""
+ps = swept(64, 48)
+prm = M.tgv2_params(niters=4, warps=1)
+ps.TGVext(prm, start=1)
+ps.set_reference(images({w}, {h}, 1)[0], I, zero)
+refused(lambda: ps.TGV(niters=4, warps=1))          # the sources are still of the old size
+refused(lambda: ps.TGVext(prm, start=0))
+sources(ps, {w}, {h})
+refused(lambda: ps.TGVext(prm, start=1))            # and the sweep's depthmap is
+ps.TGV(niters=4, warps=1)                           # from 1: nothing of the old size
+ps.TGVext(prm, start=2, u_init=np.ones(({h}, {w}), np.float32))
+ps.RunAlgorithm()
+ps.TGVext(prm, start=1)
+""")
