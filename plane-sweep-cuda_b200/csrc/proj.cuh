@@ -58,7 +58,7 @@ __device__ __forceinline__ void project_tie(double s, double g, double y, const 
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         double v = x[i] * r;
-        v = fma(fma(-v, d, x[i]), r, v);
+        v = fma(fma(v, d, -x[i]), -r, v);   // the sign of a zero stays, as below
         if (tie_distance(v) <= 64u || (unsigned)__double2hiint(v) * 2u - 1u < 2u * kNormalHi - 1u) sure = false;
         out[i] = (float)v;
     }
@@ -112,7 +112,9 @@ __device__ __forceinline__ void project(const double (&s)[M], const double (&x)[
 #pragma unroll
         for (int i = 0; i < N; ++i) {
             double v = x[m][i] * r[m];
-            v = fma(fma(-v, d[m], x[m][i]), r[m], v);   // the last place of a double
+            // the last place of a double; the negated residual of a zero x has the other
+            // sign than x, so the sum keeps x's
+            v = fma(fma(v, d[m], -x[m][i]), -r[m], v);
             tie[m] = min(tie[m], tie_distance(v));
             small = min(small, (unsigned)__double2hiint(v) * 2u - 1u);
             out[m][i] = (float)v;
