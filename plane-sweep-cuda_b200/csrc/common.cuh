@@ -123,9 +123,17 @@ cudaError_t allow_shared_memory(K *kernel, size_t most)
 // scheduled while the previous kernel of its stream is still finishing, which
 // hides the gap between the two launches (about 2.6 us per launch measured on
 // the B200).  Such a kernel calls wait_for_previous_grid() before it reads or
-// writes any global memory that the previous kernels of the stream touch: the
-// wait returns once those grids have completed and their writes are visible.
+// writes any global memory that the previous kernel of the stream touches: the
+// wait returns once that grid has completed and its writes are visible.
 // Without the launch attribute the wait returns at once.
+//
+// A kernel calls allow_next_grid() after its own wait, never before.  So when a
+// grid starts, the previous one has passed its wait: everything before that
+// previous grid is complete.  On this rests the one exception, in the kernels that
+// run several iterations per launch (tvl1_block_kernel, sparse_block_kernel,
+// tgv2_block_kernel): except in the first launch of a run, they read data that
+// was finished before the previous launch (the set-up's, which no launch of the run
+// writes) ahead of the wait.  A trigger moved before the wait would break that.
 __device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_next_grid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -437,7 +437,7 @@ dim3 slab_grid(int vw, int vh, int vd, int zb = 1)
 int slices_per_thread(int vw, int vh, int vd)
 {
     const dim3 g = slab_grid(vw, vh, vd);
-    return (size_t)g.x * g.y * g.z >= 2 * 8 * 148 ? 2 : 1;
+    return (size_t)g.x * g.y * g.z >= (size_t)2 * 8 * kSMs ? 2 : 1;
 }
 
 }  // namespace

@@ -303,7 +303,7 @@ struct PlaneSweepImpl {
                           cudaStream_t st)
     {
         const size_t n = out.elements();
-        mvs::depth_to_u8_kernel<<<(unsigned)std::min<size_t>((n + 255) / 256, 4 * 148), 256, 0, st>>>(
+        mvs::depth_to_u8_kernel<<<(unsigned)std::min<size_t>((n + 255) / 256, 4 * mvs::kSMs), 256, 0, st>>>(
             map.as<float>(), n, znear, zfar, depth8.as<uint8_t>());
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(out.data(), map.p, n * 4, cudaMemcpyDeviceToHost, st);

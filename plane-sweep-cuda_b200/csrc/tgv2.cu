@@ -721,7 +721,7 @@ __global__ void __launch_bounds__(32 * TGW) tgv2_block_kernel(BlockBufs b)
             }
     }
     if (!b.first) wait_for_previous_grid();   // dependent launch: the previous iterations are complete
-    allow_next_grid();
+    allow_next_grid();   // after the wait: the next launch reads the constant data before its own
     if (b.ctl && b.ctl->done) return;   // the run stopped at an earlier energy check
     float2 ub[RPT], vxb[RPT], vyb[RPT];
     float px[RPT][2], py[RPT][2], qx[RPT][2], qy[RPT][2], qz[RPT][2];
@@ -1556,7 +1556,7 @@ __global__ void __launch_bounds__(32 * SPW) sparse_block_kernel(SparseBufs b)
             }
     }
     if (!b.first) wait_for_previous_grid();   // dependent launch: the previous iterations are complete
-    allow_next_grid();
+    allow_next_grid();   // after the wait: the next launch reads the constant data before its own
     float u[RPT][2], vx[RPT][2], vy[RPT][2], px[RPT][2], py[RPT][2], qx[RPT][2], qy[RPT][2], qz[RPT][2];
 #pragma unroll
     for (int j = 0; j < RPT; ++j)

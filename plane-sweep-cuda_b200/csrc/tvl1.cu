@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(32 * MAXWARPS) tvl1_block_kernel(Bufs b)
         for (int k = 0; k < 3; ++k) sT[(k * rows + RPT * warp + j) * 32 + lane] = t[k];   // read by this thread only
     }
     if (!b.first) wait_for_previous_grid();   // dependent launch: the previous iterations are complete
-    allow_next_grid();
+    allow_next_grid();   // after the wait: the next launch reads the set-up's data before its own
 #pragma unroll
     for (int j = 0; j < RPT; ++j)
 #pragma unroll
