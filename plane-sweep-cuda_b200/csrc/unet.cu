@@ -43,6 +43,7 @@ constexpr int HW_ = TW + 2, HH_ = TH + 2;     // halo
 constexpr int HALO_PIX = HW_ * HH_;           // 180
 constexpr int HALO_BYTES = 2 * HALO_PIX * 16; // two 8-channel planes
 constexpr int CONV_THREADS = 128;
+constexpr int kSmemSM = 228 * 1024, kSmemReserved = 1024;   // shared memory of an SM, and of it per CTA
 // output tiles per CTA of the convolution at 16 and 32 output channels
 constexpr int CONV_MT16 = 2, CONV_MT32 = 2;
 
@@ -223,9 +224,12 @@ struct ConvSmem {
     static constexpr int TMEM_COLS = MT * COUT <= 32 ? 32 : MT * COUT <= 64 ? 64 : MT * COUT <= 128 ? 128 : 256;
 };
 
+// CTAs per SM that the registers are bounded for, by stages of the ring.
+constexpr int conv_min_ctas(int stages) { return stages == 1 ? 12 : stages == 2 ? 6 : 4; }
+
 // NST: stages of the ring, at most the number of 16-channel slices.
 template <int COUT, int MT, int NST>
-__global__ void __launch_bounds__(CONV_THREADS, NST == 1 ? 12 : NST == 2 ? 6 : 4) conv3x3_tc_kernel(ConvArgs a)
+__global__ void __launch_bounds__(CONV_THREADS, conv_min_ctas(NST)) conv3x3_tc_kernel(ConvArgs a)
 {
     using S = ConvSmem<COUT, MT>;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -443,17 +447,29 @@ int launch_conv_n(const ConvArgs &a, int B, cudaStream_t st)
     return MVS_OK;
 }
 
-// A ring of three stages, or as many as there are 16-channel slices: more CTAs
-// then share an SM.  Against two stages whose copies were waited for slice by
-// slice (batch 4, with the weight pack, B200): 192->64 at 160x120 47 -> 37 us,
-// 64->64 26 -> 22 us, 96->32 at 320x240 54 -> 47 us; one slice, 16->16 at
-// 640x480, 40 -> 37 us (fewer instructions per copied byte).
+// Stages of the ring: at most the 16-channel slices, two or three.  A third stage
+// hides more of a slice's copies, but leaves fewer CTAs per SM, and those hide them
+// too: it is taken only where the grid needs no more waves for it.  Batch 4, with the
+// weight pack, three and two stages (B200): 48->16 at 640x480 76 and 66 us, 128->128
+// at 320x240 171 and 123 us, 96->32 43 and 40 us, 128->128 at 80x60 (160 CTAs, one or
+// two per SM) 22 and 16 us; with equal waves 192->64 at 160x120 34 and 39 us, 64->64
+// at 320x240, batch 2, 26.0 and 26.8 us.  One slice, 16->16 at 640x480: 37 us.
+template <int COUT, int MT, int NST>
+int conv_waves(long long ctas)
+{
+    using S = ConvSmem<COUT, MT>;
+    const int per_sm = std::min({kSmemSM / (S::bytes(NST) + kSmemReserved), 512 / S::TMEM_COLS, conv_min_ctas(NST)});
+    return (int)((ctas + kSMs * per_sm - 1) / (kSMs * per_sm));
+}
+
 template <int COUT, int MT = 1>
 int launch_conv_t(const ConvArgs &a, int B, cudaStream_t st)
 {
     static_assert(ConvSmem<COUT, MT>::bytes(3) <= kSmemMax, "three stages fit a CTA");
+    const long long ctas = (long long)a.tiles_x * ceil_div(a.H, MT * TH) * B;
     if (a.cin <= 16) return launch_conv_n<COUT, MT, 1>(a, B, st);
-    if (a.cin <= 32) return launch_conv_n<COUT, MT, 2>(a, B, st);
+    if (a.cin <= 32 || conv_waves<COUT, MT, 3>(ctas) > conv_waves<COUT, MT, 2>(ctas))
+        return launch_conv_n<COUT, MT, 2>(a, B, st);
     return launch_conv_n<COUT, MT, 3>(a, B, st);
 }
 
@@ -502,7 +518,6 @@ constexpr int WG_COPY = 256, WG_TC_THREADS = WG_COPY + 32;   // eight copying wa
 constexpr int WG_NC = 16;                                      // input channels of a chunk, or 2 or 3 times as many
 constexpr int WG_HALO_W = TW + 2, WG_HALO_H = TH + 2;          // 10 x 18 input pixels around an 8 x 16 tile
 constexpr int WG_HALO_BYTES = 2 * WG_HALO_H * WG_HALO_W * 16;  // 5760 per 16 channels
-constexpr int WG_SMEM_SM = 228 * 1024;   // shared memory of an SM, 1 KB of it reserved per CTA
 constexpr int WG_MAX_STAGES = 8;
 // tiles a CTA sums at least: each adds its 9 x 16 x cout sums to dW atomically
 constexpr int WG_MIN_TILES = 8;
@@ -774,7 +789,7 @@ int launch_wgrad_tc_t(WgArgs a, cudaStream_t st)
 template <int M, int NC>
 int launch_wgrad_tc_m(const WgArgs &a, cudaStream_t st)
 {
-    const int room = (NC == WG_NC ? WG_SMEM_SM / 2 : WG_SMEM_SM) - 1024;
+    const int room = (NC == WG_NC ? kSmemSM / 2 : kSmemSM) - kSmemReserved;
     int r = WG_MAX_STAGES;
     while (r > 2 && wg_layout(M, r, std::min(a.cout, M) >> 3, NC).bytes > room) --r;
     switch (r) {
