@@ -44,7 +44,7 @@ UNIT = "Mpix*planes/s"
 # dram__bytes_write.sum; the TGV2 iteration also with --no-tgv-sparse, launch 51: ncu runs every
 # launch with a cold L2, so that figure is the whole working set, which stays in L2 between the
 # back-to-back iterations of a run)
-NCU_TRAFFIC = {"sweep_aggregated_kernel": 51.70432e6 + 128.86656e6,
+NCU_TRAFFIC = {"sweep_aggregated_kernel": 44.06144e6 + 132.923648e6,   # the same frame, profiles/sweep_aggregated_kernel_c2.md
                "wta_volume_kernel": 157.294336e6 + 3.661312e6,
                "tgv2_iteration_kernel": 47.945216e6 + 0.405248e6}
 # algorithmic FP32 operations per (pixel, plane, view) evaluation of the fused sweep: homography
@@ -263,7 +263,7 @@ SPARSE_BYTES_PER_PIXEL_ITERATION = 84   # u, v(2), p(2), q(3) read and written +
 
 def run_tgv_sparse(fr, dev, d_ref, wta_depth, peak_gbs, reference_gpu):
     """PlaneSweep::TGVdenoiseFromSparse on the bench frame: TGV2 from the WTA depth towards a
-    seeded 5% sample of the true depth, 200 iterations, one fused launch per iteration; beside
+    seeded 5% sample of the true depth, 200 iterations, several per launch; beside
     it the reference's own three launches per iteration on this GPU."""
     import torch
     import mvs_b200 as M
